@@ -62,7 +62,8 @@ _CUDA_SIGNATURES = {
     "msb_swiglu_bwd": (_I, [_P, _P, _P, _L, _I, _P]),
     "msb_gelu": (_I, [_P, _P, _P, _P, _L, _I, _I, _P]),
     "msb_ce_stats": (_I, [_P, _P, _P, _L, _I, _L, _I, _I, _P]),
-    "msb_ce_grad": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _L, _I, _I, _I, _I, _P]),
+    "msb_ce_mean": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _L, _I, _I, _P]),
+    "msb_ce_grad": (_I, [_P, _P, _P, _P, _P, _P, _P, _L, _I, _L, _I, _I, _I, _I, _P]),
     "msb_adamw": (_I, [_P, _P, _P, _P, _I, _P, _L, _P, _P, _P]),
     "msb_momentum": (_I, [_P, _P, _P, _I, _P, _L, _P, _P, _P]),
     "msb_sumsq_finite": (_I, [_P, _I, _L, _P, _P, _P]),

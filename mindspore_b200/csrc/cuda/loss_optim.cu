@@ -28,19 +28,98 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
   m = nm;
 }
 
+// A row as a misaligned head, whole 16-byte vectors and a tail: rows of an odd vocabulary start anywhere.
+template <typename T>
+struct CeRow {
+  static constexpr int kVec = 16 / sizeof(T);
+  int head, vecs;      // elements before the first 16-byte boundary, vectors behind it
+  __device__ __forceinline__ CeRow(const T* p, int V) {
+    const int off = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 15) / static_cast<int>(sizeof(T));
+    head = off ? kVec - off : 0;
+    if (head > V) head = V;
+    vecs = (V - head) / kVec;
+  }
+};
+
+// Sixteen bytes of a tensor as fp32 values, and back.
+__device__ __forceinline__ void unpack16(const uint4& r, float (&f)[8], __nv_bfloat16) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ void unpack16(const uint4& r, float (&f)[4], float) {
+  f[0] = __uint_as_float(r.x); f[1] = __uint_as_float(r.y); f[2] = __uint_as_float(r.z); f[3] = __uint_as_float(r.w);
+}
+__device__ __forceinline__ uint4 pack16(const float (&f)[8], __nv_bfloat16) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+__device__ __forceinline__ uint4 pack16(const float (&f)[4], float) {
+  return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+}
+__device__ __forceinline__ __nv_bfloat16 ce_round(float v, __nv_bfloat16) { return __float2bfloat16(v); }
+__device__ __forceinline__ float ce_round(float v, float) { return v; }
+
+// Adds N values: one rescaling of the sum for all of them.
+template <int N>
+__device__ __forceinline__ void online_add_n(float& m, float& s, const float (&f)[N]) {
+  float nm = m;
+#pragma unroll
+  for (int i = 0; i < N; ++i) nm = fmaxf(nm, f[i]);
+  if (nm == -INFINITY) {                     // nothing but -inf so far (a NaN is kept by the additions below)
+#pragma unroll
+    for (int i = 0; i < N; ++i) s += f[i] == -INFINITY ? 0.f : f[i];
+    return;
+  }
+  s *= __expf(m - nm);
+#pragma unroll
+  for (int i = 0; i < N; ++i) s += __expf(f[i] - nm);
+  m = nm;
+}
+
 // Per-row statistics over this rank's vocabulary slice [vocab_start, vocab_start+V):
 //   stats[row] = {max, sum exp(l - max), logit[label] if label in slice else 0}
+// and, if loss != nullptr (the slice is the whole vocabulary), loss[row] as in ce_grad_kernel.
+// Bound by reading the logits once.  Four 16-byte loads are in flight per thread; the scalar 2-byte loads this replaces
+// kept too few bytes in flight.
 template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
 ce_stats_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ stats,
-                int V, long long pitch, int vocab_start) {
+                float* __restrict__ loss, int V, long long pitch, int vocab_start, int ignore_index) {
+  constexpr int kVec = CeRow<T>::kVec;
   __shared__ float sm[kCeThreads / 32], ss[kCeThreads / 32];
   const long long row = blockIdx.x;
   const T* lr = logits + row * pitch;
+  const CeRow<T> part(lr, V);
   float m = -INFINITY, s = 0.f;
-  for (int c = threadIdx.x; c < V; c += kCeThreads) {
-    const float v = to_f<T>(lr[c]);
-    if (v > m) { s = s * __expf(m - v) + 1.f; m = v; } else { s += __expf(v - m); }
+  const uint4* body = reinterpret_cast<const uint4*>(lr + part.head);
+  int i = threadIdx.x;
+  for (; i + 3 * kCeThreads < part.vecs; i += 4 * kCeThreads) {
+    uint4 r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = body[i + u * kCeThreads];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float f[kVec];
+      unpack16(r[u], f, T());
+      online_add_n(m, s, f);
+    }
+  }
+  for (; i < part.vecs; i += kCeThreads) {
+    float f[kVec];
+    unpack16(body[i], f, T());
+    online_add_n(m, s, f);
+  }
+  if (threadIdx.x < part.head) {
+    const float f[1] = {to_f<T>(lr[threadIdx.x])};
+    online_add_n(m, s, f);
+  }
+  for (int c = part.head + part.vecs * kVec + threadIdx.x; c < V; c += kCeThreads) {
+    const float f[1] = {to_f<T>(lr[c])};
+    online_add_n(m, s, f);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -60,37 +139,102 @@ ce_stats_kernel(const T* __restrict__ logits, const int* __restrict__ labels, fl
     }
     if (lane == 0) {
       const int lab = labels[row] - vocab_start;
+      const float tgt = (lab >= 0 && lab < V) ? to_f<T>(lr[lab]) : 0.f;
       stats[row * 3 + 0] = m;
       stats[row * 3 + 1] = s;
-      stats[row * 3 + 2] = (lab >= 0 && lab < V) ? to_f<T>(lr[lab]) : 0.f;
+      stats[row * 3 + 2] = tgt;
+      if (loss) loss[row] = labels[row] != ignore_index ? (__logf(s) + m - tgt) : 0.f;
+    }
+  }
+}
+
+// mean = sum of loss over the rows / number of rows whose label is not ignored (at least 1); count = that number.
+// One block: the sums run in a fixed order.
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ loss, const int* __restrict__ labels, float* __restrict__ mean,
+               float* __restrict__ count, long long rows, int ignore_index) {
+  __shared__ float sl[32];
+  __shared__ int sn[32];
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  int n = 0;
+  long long i = threadIdx.x;
+  for (; i + 3 * 1024 < rows; i += 4 * 1024) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      acc[u] += loss[i + u * 1024];
+      n += labels[i + u * 1024] != ignore_index;
+    }
+  }
+  for (; i < rows; i += 1024) {
+    acc[0] += loss[i];
+    n += labels[i] != ignore_index;
+  }
+  const float a = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  n = __reduce_add_sync(0xffffffffu, n);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) { sl[warp] = a; sn[warp] = n; }
+  __syncthreads();
+  if (warp == 0) {
+    const float t = warp_sum(sl[lane]);
+    const int c = __reduce_add_sync(0xffffffffu, sn[lane]);
+    if (lane == 0) {
+      const float valid = static_cast<float>(c < 1 ? 1 : c);
+      *mean = t / valid;
+      *count = valid;
     }
   }
 }
 
 // Given (possibly cross-rank combined) stats, writes loss[row] = log(sum) + max - target (0 for ignored
-// rows) and, if dlogits != nullptr, dlogits = (softmax - onehot) * grad_scale[0] * (row valid).
+// rows) and, if dlogits != nullptr, dlogits = (softmax - onehot) * grad_scale[0] / (divisor ? divisor[0] : 1) * (row
+// valid).  Bound by reading and writing the logits once: 16-byte accesses, four loads in flight per thread.  Where the
+// two rows are not equally aligned every element goes by itself.
 template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
-ce_grad_kernel(const T* __restrict__ logits, const int* __restrict__ labels, const float* __restrict__ stats,
-               float* __restrict__ loss, T* __restrict__ dlogits, const float* __restrict__ grad_scale, int V,
-               long long pitch, int vocab_start, int ignore_index, int write_loss) {
+ce_grad_kernel(const T* logits, const int* __restrict__ labels, const float* __restrict__ stats,
+               float* __restrict__ loss, T* dlogits, const float* __restrict__ grad_scale,
+               const float* __restrict__ divisor, int V, long long pitch, int vocab_start, int ignore_index,
+               int write_loss) {
+  constexpr int kVec = CeRow<T>::kVec;
   const long long row = blockIdx.x;
   const float m = stats[row * 3 + 0], s = stats[row * 3 + 1], tgt = stats[row * 3 + 2];
   const int label = labels[row];
   const bool valid = label != ignore_index;
   if (threadIdx.x == 0 && write_loss) loss[row] = valid ? (__logf(s) + m - tgt) : 0.f;
   if (!dlogits) return;
-  const float scale = valid ? grad_scale[0] : 0.f;
+  const float scale = valid ? (divisor ? grad_scale[0] / divisor[0] : grad_scale[0]) : 0.f;
   const float inv = 1.f / s;
   const int lab = label - vocab_start;
   const T* lr = logits + row * pitch;
   T* dr = dlogits + row * pitch;
-  for (int c = threadIdx.x; c < V; c += kCeThreads) {
-    float g = __expf(to_f<T>(lr[c]) - m) * inv;
+  auto one = [&](float v, int c) {
+    float g = __expf(v - m) * inv;
     if (c == lab) g -= 1.f;
-    g *= scale;
-    if constexpr (sizeof(T) == 2) dr[c] = __float2bfloat16(g); else dr[c] = g;
+    return g * scale;
+  };
+  CeRow<T> part(lr, V);
+  if (((reinterpret_cast<uintptr_t>(lr) ^ reinterpret_cast<uintptr_t>(dr)) & 15) != 0) part.head = part.vecs = 0;
+  const uint4* body = reinterpret_cast<const uint4*>(lr + part.head);
+  uint4* dbody = reinterpret_cast<uint4*>(dr + part.head);
+  auto vec = [&](const uint4& r, int i) {
+    float f[kVec];
+    unpack16(r, f, T());
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) f[j] = one(f[j], part.head + i * kVec + j);
+    dbody[i] = pack16(f, T());
+  };
+  int i = threadIdx.x;
+  for (; i + 3 * kCeThreads < part.vecs; i += 4 * kCeThreads) {
+    uint4 r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = body[i + u * kCeThreads];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) vec(r[u], i + u * kCeThreads);
   }
+  for (; i < part.vecs; i += kCeThreads) vec(body[i], i);
+  if (threadIdx.x < part.head) dr[threadIdx.x] = ce_round(one(to_f<T>(lr[threadIdx.x]), threadIdx.x), T());
+  for (int c = part.head + part.vecs * kVec + threadIdx.x; c < V; c += kCeThreads)
+    dr[c] = ce_round(one(to_f<T>(lr[c]), c), T());
 }
 
 // ------------------------------------------------------------------------------------ optimizers
@@ -285,30 +429,46 @@ static inline int grid_for(long long n, int threads, int per_sm = 8) {
 
 using namespace msb;
 
+template <typename T>
+static void launch_ce_stats(const void* logits, const int* labels, float* stats, float* loss, long long rows, int V,
+                            long long pitch, int vocab_start, int ignore_index, cudaStream_t stream) {
+  ce_stats_kernel<T><<<(unsigned)rows, kCeThreads, 0, stream>>>(static_cast<const T*>(logits), labels, stats, loss, V,
+                                                                 pitch, vocab_start, ignore_index);
+}
+
 MSB_EXPORT int msb_ce_stats(const void* logits, const int* labels, float* stats, long long rows, int V,
                             long long pitch, int vocab_start, int logits_fp32, void* stream) {
   if (rows <= 0) return kOk;
-  if (logits_fp32)
-    ce_stats_kernel<float><<<(unsigned)rows, kCeThreads, 0, (cudaStream_t)stream>>>((const float*)logits, labels,
-                                                                                    stats, V, pitch, vocab_start);
-  else
-    ce_stats_kernel<__nv_bfloat16><<<(unsigned)rows, kCeThreads, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)logits, labels, stats, V, pitch, vocab_start);
+  (logits_fp32 ? launch_ce_stats<float> : launch_ce_stats<__nv_bfloat16>)(logits, labels, stats, nullptr, rows, V, pitch,
+                                                                          vocab_start, 0, (cudaStream_t)stream);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
 
+// Forward of the mean loss over a whole vocabulary in two launches: stats [rows][3] and loss [rows] as above,
+// mean = the mean over the rows that are not ignored, count = how many they are (at least 1).
+MSB_EXPORT int msb_ce_mean(const void* logits, const int* labels, float* stats, float* loss, float* mean, float* count,
+                           long long rows, int V, long long pitch, int ignore_index, int logits_fp32, void* stream) {
+  if (rows > 0)
+    (logits_fp32 ? launch_ce_stats<float> : launch_ce_stats<__nv_bfloat16>)(logits, labels, stats, loss, rows, V, pitch,
+                                                                            0, ignore_index, (cudaStream_t)stream);
+  ce_mean_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(loss, labels, mean, count, rows, ignore_index);
+  MSB_CUDA_CHECK(cudaGetLastError());
+  return kOk;
+}
+
+// divisor (may be null): one more device scalar that the gradient is divided by.
 MSB_EXPORT int msb_ce_grad(const void* logits, const int* labels, const float* stats, float* loss, void* dlogits,
-                           const float* grad_scale, long long rows, int V, long long pitch, int vocab_start,
-                           int ignore_index, int write_loss, int logits_fp32, void* stream) {
+                           const float* grad_scale, const float* divisor, long long rows, int V, long long pitch,
+                           int vocab_start, int ignore_index, int write_loss, int logits_fp32, void* stream) {
   if (rows <= 0) return kOk;
   if (logits_fp32)
     ce_grad_kernel<float><<<(unsigned)rows, kCeThreads, 0, (cudaStream_t)stream>>>(
-        (const float*)logits, labels, stats, loss, (float*)dlogits, grad_scale, V, pitch, vocab_start, ignore_index,
-        write_loss);
+        (const float*)logits, labels, stats, loss, (float*)dlogits, grad_scale, divisor, V, pitch, vocab_start,
+        ignore_index, write_loss);
   else
     ce_grad_kernel<__nv_bfloat16><<<(unsigned)rows, kCeThreads, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)logits, labels, stats, loss, (__nv_bfloat16*)dlogits, grad_scale, V, pitch,
+        (const __nv_bfloat16*)logits, labels, stats, loss, (__nv_bfloat16*)dlogits, grad_scale, divisor, V, pitch,
         vocab_start, ignore_index, write_loss);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;

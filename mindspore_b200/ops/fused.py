@@ -303,19 +303,18 @@ class _SoftmaxCEFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, logits, labels, ignore_index):
-        labels = labels.reshape(-1).to(torch.int32)
-        stats = K.ce_stats(logits, labels)
-        loss_rows, _ = K.ce_loss_grad(logits, labels, stats, None, ignore_index=ignore_index, want_grad=False)
-        nvalid = (labels != ignore_index).sum().clamp(min=1).float()
-        ctx.save_for_backward(logits, labels, stats, nvalid)
+        labels = labels.reshape(-1).to(torch.int32).contiguous()
+        loss, stats, count = K.ce_mean(logits, labels, ignore_index)
+        ctx.save_for_backward(logits, labels, stats, count)
         ctx.ignore_index = ignore_index
-        return loss_rows.sum() / nvalid
+        return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        logits, labels, stats, nvalid = ctx.saved_tensors
-        scale = (dloss.float() / nvalid).reshape(1).contiguous()
-        _, dl = K.ce_loss_grad(logits, labels, stats, scale, ignore_index=ctx.ignore_index, want_grad=True)
+        logits, labels, stats, count = ctx.saved_tensors
+        scale = dloss.float().reshape(1).contiguous()
+        _, dl = K.ce_loss_grad(logits, labels, stats, scale, ignore_index=ctx.ignore_index, divisor=count,
+                               want_loss=False)
         return dl.view(logits.shape), None, None
 
 

@@ -264,18 +264,35 @@ def ce_stats(logits, labels, vocab_start=0):
     return stats
 
 
-def ce_loss_grad(logits, labels, stats, grad_scale, vocab_start=0, ignore_index=-100, dlogits=None,
-                 want_grad=True):
-    """Per-row loss and (optionally) in-place-able dlogits = (softmax - onehot) * grad_scale[0]."""
+def ce_mean(logits, labels, ignore_index=-100):
+    """Mean loss over the rows whose label is not ``ignore_index``, in two launches.  Returns (loss [], stats [rows, 3],
+    count [1]): count is the number of rows the loss is a mean of (at least 1)."""
     V = logits.shape[-1]
     rows = logits.numel() // V
     l2 = logits.reshape(rows, V)
-    loss = torch.empty(rows, dtype=f32, device=logits.device)
+    stats = torch.empty(rows, 3, dtype=f32, device=logits.device)
+    row_loss = torch.empty(rows, dtype=f32, device=logits.device)
+    mean = torch.empty((), dtype=f32, device=logits.device)
+    count = torch.empty(1, dtype=f32, device=logits.device)
+    rc = _native.cuda().msb_ce_mean(_p(l2), _p(labels), _p(stats), _p(row_loss), _p(mean), _p(count), rows, V,
+                                    l2.stride(0), ignore_index, int(logits.dtype == f32), _stream())
+    _native.check(rc, "ce_mean")
+    _count(2)
+    return mean, stats, count
+
+
+def ce_loss_grad(logits, labels, stats, grad_scale, vocab_start=0, ignore_index=-100, dlogits=None,
+                 want_grad=True, divisor=None, want_loss=True):
+    """Per-row loss and (optionally) in-place-able dlogits = (softmax - onehot) * grad_scale[0] (/ divisor[0])."""
+    V = logits.shape[-1]
+    rows = logits.numel() // V
+    l2 = logits.reshape(rows, V)
+    loss = torch.empty(rows, dtype=f32, device=logits.device) if want_loss else None
     if want_grad and dlogits is None:
         dlogits = torch.empty_like(l2)
     rc = _native.cuda().msb_ce_grad(_p(l2), _p(labels), _p(stats), _p(loss), _p(dlogits) if want_grad else None,
-                                    _p(grad_scale), rows, V, l2.stride(0), vocab_start, ignore_index, 1,
-                                    int(logits.dtype == f32), _stream())
+                                    _p(grad_scale), _p(divisor), rows, V, l2.stride(0), vocab_start, ignore_index,
+                                    int(want_loss), int(logits.dtype == f32), _stream())
     _native.check(rc, "ce_grad")
     _count()
     return loss, dlogits

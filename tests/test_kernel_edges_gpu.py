@@ -1,0 +1,71 @@
+"""Kernels at the sizes where they can go wrong - edges of tiles, ragged remainders, the smallest and largest of a range -
+against fp64 / fp32 PyTorch.  Tolerances: 2^-9 is half a unit in the last place of bf16 relative to the largest value
+(fp16: 2^-12); a result that is rounded k times on its way may be off by k such steps."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+ULP = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12, torch.float32: 2.0 ** -24}
+
+
+@pytest.fixture(scope="module")
+def K():
+    from mindspore_b200 import _native
+    from mindspore_b200.ops import kernels
+    assert _native.cuda() is not None, "native CUDA library is not loaded"
+    torch.manual_seed(3)
+    return kernels
+
+
+def _near(got, exp, steps, dtype, rel=True):
+    """Largest difference within ``steps`` roundings of the largest value."""
+    got, exp = got.double(), exp.double()
+    bound = steps * ULP[dtype] * (exp.abs().max().item() if rel else 1.0)
+    assert torch.isfinite(got).all()
+    err = (got - exp).abs().max().item()
+    assert err <= bound, "error %g, bound %g" % (err, bound)
+
+
+def _status_ok():
+    from mindspore_b200 import _native
+    torch.cuda.synchronize()
+    assert _native.device_status() == 0
+
+
+# ------------------------------------------------------------------------------------------------ cross entropy
+@pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (5, 4099), (64, 32000), (9, 50257)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_cross_entropy_ragged_vocabulary(K, rows, V, dtype):
+    """Vocabularies that leave rows misaligned, ignored rows, -inf logits, an in-place gradient."""
+    from mindspore_b200.ops import fused
+    x = (2 * torch.randn(rows, V, device=DEV)).to(dtype)
+    if V > 100:
+        x[:, 3::5] = -math.inf
+    lab = torch.randint(0, V, (rows, 2), device=DEV, dtype=torch.int32)[:, 0]
+    lab[lab % 5 == 3] -= 1
+    lab[1::4] = -100
+    a = x.clone().requires_grad_(True)
+    loss = fused.softmax_cross_entropy(a, lab)
+    (3 * loss).backward()
+    r = x.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(r, lab.long())
+    (3 * ref).backward()
+    assert abs(float(loss) - float(ref)) <= 1e-5 * max(1.0, abs(float(ref)))
+    _near(a.grad, r.grad, 2 if dtype == torch.bfloat16 else 256, dtype)      # fp32: exp of the fast unit
+    st = K.ce_stats(a.detach(), lab.contiguous())
+    buf = x.clone()
+    K.ce_loss_grad(buf, lab.contiguous(), st, torch.full((1,), 0.5, device=DEV), dlogits=buf)
+    valid = int((lab != -100).sum())
+    _near(buf, r.grad * (0.5 * valid / 3), 2 if dtype == torch.bfloat16 else 256, dtype)
+
+
+def test_cross_entropy_without_a_valid_row(K):
+    from mindspore_b200.ops import fused
+    x = torch.randn(4, 40, device=DEV).bfloat16().requires_grad_(True)
+    loss = fused.softmax_cross_entropy(x, torch.full((4,), -100, device=DEV, dtype=torch.int32))
+    loss.backward()
+    assert float(loss) == 0 and not x.grad.any()
