@@ -24,6 +24,60 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// Packed pairs of fp32 values: one instruction for two elements.
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// D[tmem] (+)= A[tmem] * B[smem desc]: the 16-bit A operand lies in tensor memory, lane = row, two consecutive k per
+// 32-bit column.
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// One arrival for the whole warp: 128 or 256 single arrivals on one barrier word are served one after the other.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+
+// Item of this CTA in round r of a persistent loop over items sorted by falling length: CTAs take items in turn, every
+// second round in reverse order, so that the CTA with the longest item of one round gets the shortest of the next
+// (causal, 512 items on 148 CTAs: longest CTA at 1.04 of the mean instead of 1.29).  The first value beyond the last
+// item ends the loop: only the last round can reach beyond it.
+__device__ __forceinline__ int fa_snake(int round) {
+  const int g = gridDim.x, c = blockIdx.x;
+  return round * g + ((round & 1) ? g - 1 - c : c);
+}
+
 // Loads a [rows x 128] bf16 tile of head h starting at token t0 as two 128B-swizzled halves
 // (d 0..63 at dst, d 64..127 at dst + rows*128 bytes).
 __device__ __forceinline__ void fa_load_tile(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int rows, int h,

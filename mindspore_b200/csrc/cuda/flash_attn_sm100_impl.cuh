@@ -1,17 +1,31 @@
 // FlashAttention forward for sm_100a (head_dim 128, bf16, causal or full), tcgen05 + TMEM + TMA.
 //
 // Tensors are token-major: q[b][s][h][d], k/v[b][s][hk][d], o[b][s][h][d]; row pitches are parameters so
-// q/k/v may be column slices of one fused QKV GEMM output.  One work item = (batch, head, 128 query rows).
+// q/k/v may be column slices of one fused QKV GEMM output.  One work item = (batch, head, 256 query rows): two
+// tiles of 128 rows that share every K and V tile.
 //
-// Persistent CTA, 192 threads:
-//   warp 0    : TMA producer  (Q once per item; K and V tiles of 128 keys, double-buffered)
-//   warp 1    : MMA issuer    S[buf] = Q K^T into TMEM (double-buffered, so QK of block j+1 overlaps the
-//                             softmax of block j), then O += P V
-//   warps 2-5 : softmax       thread t owns query row t: reads its S row from TMEM (no shuffles), keeps the
-//                             running max / sum, writes P (bf16) into 128B-swizzled shared memory as the A
-//                             operand of the PV MMA, rescales O in TMEM only when the row max grew by more
-//                             than 2^8 (warp-uniform decision), and finally normalises and stores O and LSE.
-// TMEM: S0 [0,128) S1 [128,256) O [256,384) of a 512-column allocation.
+// Persistent CTA, 384 threads (three warpgroups; the first gives most of its registers to the other two):
+//   warp 0    : TMA producer  (both Q tiles once per item; K and V tiles of 128 keys through one ring of four)
+//   warp 1    : MMA issuer    per key block and tile: O_t += P_t V, then S_t = Q_t K^T of the next block
+//   warps 2-3 : idle
+//   warps 4-7 : softmax of tile 0, warps 8-11 : softmax of tile 1.  Thread t owns query row t of its tile: reads its S
+//                             row from TMEM (no shuffles), keeps the running max / sum, writes P (16-bit) back into
+//                             the first 64 columns of the S row it came from, where the P V product reads it as its
+//                             TMEM operand; rescales O in TMEM only when the row max grew by more than 2^8
+//                             (warp-uniform decision), and finally normalises and stores O and LSE.
+// TMEM: S0 / P0 [0,128)  S1 / P1 [128,256)  O0 [256,384)  O1 [384,512).
+//
+// Why this split.  The exponentials (16 per cycle per SM: 1024 cycles per 128 x 128 tile) and the two products of a
+// tile (1024 cycles) take equally long, so they have to run at the same time: while one tile's softmax runs, the
+// tensor core works for the other tile.  One tile per CTA with P going through shared memory (the earlier form of this
+// kernel) left the tensor pipe idle for two thirds of the time.  All products of a CTA are issued by one thread and
+// execute in issue order, which is what orders "S_t of the next block overwrites P_t" behind "P_t V has read it".
+//
+// Measured, 2 x 4096 tokens x 32 heads, bf16: causal 0.41 -> 0.27 ms (1030 TFLOP/s), full 0.74 -> 0.49 ms (1124); 0.35 and
+// 0.58 ms while a lone lane issued the products (see elect_one).  What bounds it now are the products: with the softmax's
+// arithmetic left out the full case still takes 0.43 ms.  Q K^T reads 8 KB of shared memory per 64 cycles, all that an SM
+// can, and the TMA's writes come on top.  Moving a quarter to a half of the exponentials to the FMA pipe (degree-5
+// polynomial) cost 5 to 11 %, handing the first half of P to the tensor core early 7 %.
 //
 // The reference defines FlashAttentionScore (core/ops/ops_def/flash_attention_score_op.yaml) but ships no GPU
 // kernel for it; its GPU path would be BatchMatMul + Softmax + BatchMatMul through cuBLAS/cuDNN.
@@ -23,9 +37,10 @@
 namespace msb {
 namespace MSB_ELEM_NS {
 
-constexpr int kFaBM = 128;       // query rows per item
+constexpr int kFaBM = 128;       // query rows per tile
 constexpr int kFaBN = 128;       // keys per block
-constexpr int kFaThreads = 192;
+constexpr int kFaThreads = 384;
+constexpr int kFaRing = 4;       // K / V tiles in flight
 constexpr int kTileBytes = 128 * 128 * 2;  // 32 KB: one 128x128 bf16 tile (two 128B-swizzled halves)
 
 struct FaParams {
@@ -39,22 +54,30 @@ struct FaParams {
   float scale;
 };
 
-// shared memory map (1024B aligned): Q 32K | K0 32K | K1 32K | V0 32K | V1 32K | P 32K | barriers
+// shared memory map (1024B aligned): Q0 32K | Q1 32K | ring of four 32K tiles | barriers
 struct FaSmem {
   static constexpr int kQ = 0;
-  static constexpr int kK = kTileBytes;
-  static constexpr int kV = 3 * kTileBytes;
-  static constexpr int kP = 5 * kTileBytes;
-  static constexpr int kBar = 6 * kTileBytes;
+  static constexpr int kRing = 2 * kTileBytes;
+  static constexpr int kBar = (2 + kFaRing) * kTileBytes;
   static constexpr int kBytes = kBar + 256 + 1024;
 };
 
-__device__ __forceinline__ void fa_item(int w, const FaParams& p, int nq, int& b, int& h, int& qb) {
+// Work item -> (batch, head, pair of query tiles, key blocks of each tile).  n1 is 0 when the second tile lies beyond
+// the sequence.
+struct FaItem {
+  int b, h, qb, n0, n1;
+};
+__device__ __forceinline__ FaItem fa_item(int w, const FaParams& p, int nq2, int nk) {
+  FaItem it;
   const int bh = p.B * p.H;
-  qb = nq - 1 - w / bh;     // longest (latest) query blocks first
+  it.qb = nq2 - 1 - w / bh;     // longest (latest) query blocks first
   const int r = w % bh;
-  b = r / p.H;
-  h = r % p.H;
+  it.b = r / p.H;
+  it.h = r % p.H;
+  const bool second = it.qb * 256 + 128 < p.S;
+  it.n0 = p.causal ? 2 * it.qb + 1 : nk;
+  it.n1 = second ? (p.causal ? 2 * it.qb + 2 : nk) : 0;
+  return it;
 }
 
 __global__ void __launch_bounds__(kFaThreads, 1)
@@ -63,38 +86,35 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FaSmem::kBar);
-  uint64_t* q_full = bars + 0;
-  uint64_t* q_empty = bars + 1;
-  uint64_t* k_full = bars + 2;    // [2]
-  uint64_t* k_empty = bars + 4;   // [2]
-  uint64_t* v_full = bars + 6;    // [2]
-  uint64_t* v_empty = bars + 8;   // [2]
-  uint64_t* s_full = bars + 10;   // [2]
-  uint64_t* s_empty = bars + 12;  // [2]
-  uint64_t* p_ready = bars + 14;
-  uint64_t* o_done = bars + 15;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* q_full = bars + 0;    // [2]
+  uint64_t* q_empty = bars + 2;   // [2]
+  uint64_t* r_full = bars + 4;    // [kFaRing]
+  uint64_t* r_empty = bars + 8;   // [kFaRing]
+  uint64_t* s_full = bars + 12;   // [2]
+  uint64_t* p_ready = bars + 14;  // [2]
+  uint64_t* o_full = bars + 16;   // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const AbortCtx ab{cta_abort, p.status};
-  const int nq = p.S / kFaBM;
-  const int total = p.B * p.H * nq;
+  const int nq2 = (p.S + 2 * kFaBM - 1) / (2 * kFaBM);
+  const int nk = (p.S + kFaBN - 1) / kFaBN;
+  const int total = p.B * p.H * nq2;
   const int group = p.H / p.Hk;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 128);
+      mbar_init(&p_ready[i], 4);
+      mbar_init(&o_full[i], 1);
     }
-    mbar_init(p_ready, 128);
-    mbar_init(o_done, 1);
+    for (int i = 0; i < kFaRing; ++i) {
+      mbar_init(&r_full[i], 1);
+      mbar_init(&r_empty[i], 1);
+    }
     *cta_abort = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmQ);
@@ -108,220 +128,237 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_o = tmem_base + 256;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  if (warp == 0) {
-    if (lane == 0) {
+  // registers: 384 threads x 168 at launch = 128 x 88 + 256 x 208 (the MMA thread spills below 88)
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp == 0 && lane == 0) {
       // ------------------------------------------------------------------ TMA producer
-      uint32_t items = 0, kvc = 0;
+      uint32_t qc[2] = {0, 0}, rc = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++items) {
-        int b, h, qb;
-        fa_item(w, p, nq, b, h, qb);
-        const int hk = h / group;
-        const int nblk = p.causal ? qb + 1 : p.S / kFaBN;
-        if (!mbar_wait(q_empty, (items & 1) ^ 1, ab)) { ok = false; break; }
-        mbar_expect_tx(q_full, kTileBytes);
-        tma_load_4d(smem + FaSmem::kQ, &tmQ, q_full, 0, h, qb * kFaBM, b);
-        tma_load_4d(smem + FaSmem::kQ + 16384, &tmQ, q_full, 64, h, qb * kFaBM, b);
-        for (int j = 0; j < nblk; ++j, ++kvc) {
-          const int st = kvc & 1;
-          const uint32_t ph = (kvc >> 1) & 1;
-          if (!mbar_wait(&k_empty[st], ph ^ 1, ab)) { ok = false; break; }
-          mbar_expect_tx(&k_full[st], kTileBytes);
-          uint8_t* kd = smem + FaSmem::kK + st * kTileBytes;
-          tma_load_4d(kd, &tmK, &k_full[st], 0, hk, j * kFaBN, b);
-          tma_load_4d(kd + 16384, &tmK, &k_full[st], 64, hk, j * kFaBN, b);
-          if (!mbar_wait(&v_empty[st], ph ^ 1, ab)) { ok = false; break; }
-          mbar_expect_tx(&v_full[st], kTileBytes);
-          uint8_t* vd = smem + FaSmem::kV + st * kTileBytes;
-          tma_load_4d(vd, &tmV, &v_full[st], 0, hk, j * kFaBN, b);
-          tma_load_4d(vd + 16384, &tmV, &v_full[st], 64, hk, j * kFaBN, b);
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc_qk = umma_idesc_elem(128, 128, false, false);
-      constexpr uint32_t idesc_pv = umma_idesc_elem(128, 128, false, true);   // V is MN-major (d contiguous)
-      const uint32_t q_addr = smem_u32(smem + FaSmem::kQ);
-      const uint32_t p_addr = smem_u32(smem + FaSmem::kP);
-      uint32_t items = 0, kvc = 0, sc = 0, pc = 0;
-      bool ok = true;
-      auto issue_qk = [&](uint32_t kv_index, uint32_t s_index) -> bool {
-        const int st = kv_index & 1;
-        const int sb = s_index & 1;
-        if (!mbar_wait(&k_full[st], (kv_index >> 1) & 1, ab)) return false;
-        if (!mbar_wait(&s_empty[sb], ((s_index >> 1) & 1) ^ 1, ab)) return false;
-        tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(smem + FaSmem::kK + st * kTileBytes);
-#pragma unroll
-        for (int kk = 0; kk < kFaD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_bf16(tmem_base + sb * 128, umma_smem_desc(q_addr + off, 16, 1024),
-                    umma_smem_desc(k_addr + off, 16, 1024), idesc_qk, kk != 0);
-        }
-        umma_commit(&s_full[sb]);
-        umma_commit(&k_empty[st]);
+      auto load_q = [&](const FaItem& it, int t) -> bool {
+        if (!mbar_wait(&q_empty[t], (qc[t] & 1) ^ 1, ab)) return false;
+        ++qc[t];
+        mbar_expect_tx(&q_full[t], kTileBytes);
+        fa_load_tile(smem + FaSmem::kQ + t * kTileBytes, &tmQ, &q_full[t], 128, it.h, it.qb * 256 + t * 128, it.b);
         return true;
       };
-      for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++items) {
-        int b, h, qb;
-        fa_item(w, p, nq, b, h, qb);
-        const int nblk = p.causal ? qb + 1 : p.S / kFaBN;
-        if (!mbar_wait(q_full, items & 1, ab)) { ok = false; break; }
-        if (!issue_qk(kvc, sc)) { ok = false; break; }
-        ++sc;
-        for (int j = 0; j < nblk; ++j) {
-          if (j + 1 < nblk) {
-            if (!issue_qk(kvc + 1 + j, sc)) { ok = false; break; }
-            ++sc;
-          } else {
-            umma_commit(q_empty);  // last QK of this item is in flight: Q may be reloaded when it retires
-          }
-          const uint32_t kv_index = kvc + j;
-          const int st = kv_index & 1;
-          if (!mbar_wait(p_ready, pc & 1, ab)) { ok = false; break; }
-          ++pc;
-          if (!mbar_wait(&v_full[st], (kv_index >> 1) & 1, ab)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t v_addr = smem_u32(smem + FaSmem::kV + st * kTileBytes);
+      auto load_kv = [&](const CUtensorMap* tm, int hk, int j, int b) -> bool {
+        const int st = rc & (kFaRing - 1);
+        if (!mbar_wait(&r_empty[st], ((rc / kFaRing) & 1) ^ 1, ab)) return false;
+        mbar_expect_tx(&r_full[st], kTileBytes);
+        fa_load_tile(smem + FaSmem::kRing + st * kTileBytes, tm, &r_full[st], 128, hk, j * kFaBN, b);
+        ++rc;
+        return true;
+      };
+      for (int round = 0, w; ok && (w = fa_snake(round)) < total; ++round) {
+        const FaItem it = fa_item(w, p, nq2, nk);
+        const int hk = it.h / group, n = it.n1 > it.n0 ? it.n1 : it.n0;
+        ok = load_q(it, 0) && load_kv(&tmK, hk, 0, it.b) && (it.n1 == 0 || load_q(it, 1)) &&
+             load_kv(&tmV, hk, 0, it.b);
+        for (int j = 1; j < n && ok; ++j) ok = load_kv(&tmK, hk, j, it.b) && load_kv(&tmV, hk, j, it.b);
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer (the whole warp, one elected lane)
+      constexpr uint32_t idesc_qk = umma_idesc_elem(128, 128, false, false);
+      constexpr uint32_t idesc_pv = umma_idesc_elem(128, 128, false, true);   // V is MN-major (d contiguous)
+      const uint32_t lead = elect_one();
+      uint32_t base = 0;              // ring index of K of block 0 of the item; K_j at base + 2j, V_j at base + 2j + 1
+      uint32_t qc[2] = {0, 0}, pc[2] = {0, 0};
+      const uint64_t q_desc = umma_smem_desc(smem_u32(smem + FaSmem::kQ), 16, 1024);
+      const uint64_t k_desc = umma_smem_desc(smem_u32(smem + FaSmem::kRing), 16, 1024);
+      const uint64_t v_desc = umma_smem_desc(smem_u32(smem + FaSmem::kRing), 16384, 1024);
+      auto wait_ring = [&](uint32_t i) -> bool {
+        const bool r = mbar_wait_warp(&r_full[i & (kFaRing - 1)], (i / kFaRing) & 1, ab);
+        tc_fence_after_sync();
+        return r;
+      };
+      auto issue_qk = [&](int t, uint32_t ki) {
+        const uint64_t qd = q_desc + t * (kTileBytes >> 4), kd = k_desc + (ki & (kFaRing - 1)) * (kTileBytes >> 4);
+        if (lead) {
 #pragma unroll
-          for (int kk = 0; kk < kFaBN / 16; ++kk) {
-            const uint64_t adesc = umma_smem_desc(p_addr + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-            const uint64_t bdesc = umma_smem_desc(v_addr + kk * 2048, 16384, 1024);
-            umma_bf16(tmem_o, adesc, bdesc, idesc_pv, (j | kk) != 0);
+          for (int kk = 0; kk < kFaD / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+            umma_bf16(tmem_base + t * 128, qd + off, kd + off, idesc_qk, kk != 0);
           }
-          umma_commit(&v_empty[st]);
-          umma_commit(o_done);
+          umma_commit(&s_full[t]);
         }
-        kvc += nblk;
+        __syncwarp();
+      };
+      auto issue_pv = [&](int t, uint32_t vi, bool first) {
+        const uint64_t vd = v_desc + (vi & (kFaRing - 1)) * (kTileBytes >> 4);
+        if (lead) {
+#pragma unroll
+          for (int kk = 0; kk < kFaBN / 16; ++kk)
+            umma_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, vd + ((kk * 2048) >> 4), idesc_pv,
+                    !(first && kk == 0));
+        }
+        __syncwarp();
+      };
+      auto commit = [&](uint64_t* bar) {
+        if (lead) umma_commit(bar);
+        __syncwarp();
+      };
+      bool ok = true;
+      for (int round = 0, w; ok && (w = fa_snake(round)) < total; ++round) {
+        const FaItem it = fa_item(w, p, nq2, nk);
+        const int n = it.n1 > it.n0 ? it.n1 : it.n0;
+        const int cnt[2] = {it.n0, it.n1};
+        ok = wait_ring(base);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (!ok || cnt[t] == 0) continue;
+          if (!(ok = mbar_wait_warp(&q_full[t], qc[t] & 1, ab))) break;
+          ++qc[t];
+          tc_fence_after_sync();
+          issue_qk(t, base);
+          if (cnt[t] == 1) commit(&q_empty[t]);
+        }
+        if (ok) commit(&r_empty[base & (kFaRing - 1)]);
+        for (int j = 0; j < n && ok; ++j) {
+          const uint32_t vi = base + 2 * j + 1, ki = base + 2 * j + 2;
+          const int last = j < it.n1 ? 1 : 0;          // the last tile that reads V_j
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (!ok || j >= cnt[t]) continue;
+            if (!(ok = wait_ring(vi))) break;
+            if (!(ok = mbar_wait_warp(&p_ready[t], pc[t] & 1, ab))) break;
+            ++pc[t];
+            tc_fence_after_sync();
+            issue_pv(t, vi, j == 0);
+            if (t == last) commit(&r_empty[vi & (kFaRing - 1)]);
+            if (j + 1 == cnt[t]) commit(&o_full[t]);
+            if (j + 1 < cnt[t]) {
+              if (!(ok = wait_ring(ki))) break;
+              issue_qk(t, ki);
+              // the last tile that reads K_{j+1} releases it; the last product with Q_t releases Q_t
+              if (t == (j + 1 < it.n1 ? 1 : 0)) commit(&r_empty[ki & (kFaRing - 1)]);
+              if (j + 2 == cnt[t]) commit(&q_empty[t]);
+            }
+          }
+        }
+        base += 2 * n;
       }
     }
     __syncwarp();
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     // -------------------------------------------------------------------- softmax / correction / epilogue
+    const int t = (warp >> 2) - 1;                 // tile
     const int q = warp & 3;
     const int row = q * 32 + lane;                 // row inside the 128-row tile == TMEM lane
     const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
-    uint8_t* p_smem = smem + FaSmem::kP;
+    const uint32_t tm_s = tmem_base + t * 128 + lane_sel;
+    const uint32_t tm_o = tmem_base + 256 + t * 128 + lane_sel;
     uint32_t sc = 0, oc = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-      int b, h, qb;
-      fa_item(w, p, nq, b, h, qb);
-      const int nblk = p.causal ? qb + 1 : p.S / kFaBN;
+    for (int round = 0, w; ok && (w = fa_snake(round)) < total; ++round) {
+      const FaItem it = fa_item(w, p, nq2, nk);
+      const int nblk = t == 0 ? it.n0 : it.n1;
+      if (nblk == 0) continue;
+      const int tile = it.qb * 2 + t;
       float m_used = -INFINITY;   // max the stored probabilities are relative to (log2 domain)
       float l = 0.f;
       for (int j = 0; j < nblk; ++j, ++sc) {
-        const int sb = sc & 1;
-        if (!mbar_wait(&s_full[sb], (sc >> 1) & 1, ab)) { ok = false; break; }
+        if (!mbar_wait(&s_full[t], sc & 1, ab)) { ok = false; break; }
         tc_fence_after_sync();
-        // raw scores; the softmax scale is folded into the exponent below (one FFMA per element) and every
-        // reduction runs on four independent accumulators: with one warp per scheduler a serial chain of 128
-        // dependent max / add instructions would cost its full latency 128 times
-        float s[128];
-        {
-          // the four loads are issued back to back and waited for once: one TMEM round trip instead of four
-          uint32_t r[4][32];
+        // raw scores; the softmax scale is folded into the exponent below (one FFMA per element)
+        uint32_t s[4][32];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld_32x32(tmem_base + sb * 128 + lane_sel + c * 32, r[c]);
-          tmem_ld_wait();
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i) s[c * 32 + i] = __uint_as_float(r[c][i]);
-        }
-        tc_fence_before_sync();
-        mbar_arrive(&s_empty[sb]);
-        if (p.causal && j == qb) {
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(tm_s + c * 32, s[c]);
+        tmem_ld_wait();
+        // keys this row may see in this block: the diagonal block is cut after the row's own key, the last block of a
+        // ragged sequence after the sequence's last key
+        int limit = p.S - j * kFaBN;
+        if (p.causal && j == tile) limit = min(limit, row + 1);
+        if ((p.causal && j == tile) || (j + 1) * kFaBN > p.S) {
 #pragma unroll
           for (int i = 0; i < 128; ++i)
-            if (i > row) s[i] = -INFINITY;
+            if (i >= limit) s[i >> 5][i & 31] = __float_as_uint(-INFINITY);
         }
-        float mx4[4] = {s[0], s[1], s[2], s[3]};
+        float mx4[4];
 #pragma unroll
-        for (int i = 4; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], s[i]);
+        for (int c = 0; c < 4; ++c) {
+          mx4[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
+#pragma unroll
+          for (int i = 2; i < 32; i += 2)
+            mx4[c] = fmaxf(fmaxf(mx4[c], __uint_as_float(s[c][i])), __uint_as_float(s[c][i + 1]));
+        }
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;   // scale > 0
         // rescale only when some row of this warp grew its max by more than 8 (in log2 units)
         const bool grow = mx > m_used + 8.f;
-        const bool warp_grow = __any_sync(0xffffffffu, grow);
-        float alpha = 1.f;
-        if (warp_grow) {
+        if (__any_sync(0xffffffffu, grow)) {
           const float m_new = fmaxf(m_used, mx);
-          alpha = (m_used == -INFINITY) ? 0.f : ex2(m_used - m_new);
+          const float alpha = (m_used == -INFINITY) ? 0.f : ex2(m_used - m_new);
           m_used = m_new;
-        }
-        const float neg_m = -m_used;
-        float rs4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int i = 0; i < 128; ++i) {
-          s[i] = ex2(fmaf(s[i], p.scale_log2, neg_m));
-          rs4[i & 3] += s[i];
-        }
-        l = l * alpha + ((rs4[0] + rs4[1]) + (rs4[2] + rs4[3]));
-        if (j > 0) {
-          // previous PV must have retired before O is rescaled or P is overwritten
-          if (!mbar_wait(o_done, oc & 1, ab)) { ok = false; break; }
-          ++oc;
-          tc_fence_after_sync();
-          if (warp_grow) {
-#pragma unroll
+          l *= alpha;
+          // S of this block was issued behind P V of the previous one: O is complete and nobody else touches it
+          if (j > 0) {
+#pragma unroll 1
             for (int c = 0; c < 4; ++c) {
               uint32_t r[32];
-              tmem_ld_32x32(tmem_o + lane_sel + c * 32, r);
+              tmem_ld_32x32(tm_o + c * 32, r);
               tmem_ld_wait();
 #pragma unroll
               for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st_32x32(tmem_o + lane_sel + c * 32, r);
+              tmem_st_32x32(tm_o + c * 32, r);
             }
-            tmem_st_wait();
           }
         }
-        // P row -> shared memory, K-major 128B swizzle: 16-byte chunk ch of row r lands at chunk (ch ^ (r & 7))
+        const uint64_t scale2 = f32x2(p.scale_log2, p.scale_log2), neg_m2 = f32x2(-m_used, -m_used);
+        uint64_t rs[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int ch = 0; ch < 16; ++ch) {
-          uint4 v;
-          v.x = pack_e2(s[ch * 8 + 0], s[ch * 8 + 1]);
-          v.y = pack_e2(s[ch * 8 + 2], s[ch * 8 + 3]);
-          v.z = pack_e2(s[ch * 8 + 4], s[ch * 8 + 5]);
-          v.w = pack_e2(s[ch * 8 + 6], s[ch * 8 + 7]);
-          const int half = ch >> 3, cc = ch & 7;
-          *reinterpret_cast<uint4*>(p_smem + half * 16384 + row * 128 + ((cc ^ (row & 7)) << 4)) = v;
+        for (int h = 0; h < 2; ++h) {
+          // pairs 2i, 2i + 1 become word i of the same register array: nothing else is needed to hold P
+#pragma unroll
+          for (int i = h * 32; i < h * 32 + 32; ++i) {
+            const uint32_t* e = &s[i >> 4][(2 * i) & 31];
+            float a, b;
+            f32x2_split(fma2(f32x2(__uint_as_float(e[0]), __uint_as_float(e[1])), scale2, neg_m2), a, b);
+            a = ex2(a);
+            b = ex2(b);
+            rs[i & 3] = add2(rs[i & 3], f32x2(a, b));
+            s[h][i & 31] = pack_e2(a, b);
+          }
+          tmem_st_32x32(tm_s + h * 32, s[h]);
         }
-        fence_proxy_async_smem();
+        tmem_st_wait();
         tc_fence_before_sync();
-        mbar_arrive(p_ready);
+        warp_arrive(&p_ready[t], lane);
+        float a, b;
+        f32x2_split(add2(add2(rs[0], rs[1]), add2(rs[2], rs[3])), a, b);
+        l += a + b;
       }
       if (!ok) break;
-      // ---- epilogue: O / l -> global, LSE
-      if (!mbar_wait(o_done, oc & 1, ab)) { ok = false; break; }
+      // ---- epilogue: O / l -> global, LSE.  The next write to O comes behind this thread's next p_ready.
+      if (!mbar_wait(&o_full[t], oc & 1, ab)) { ok = false; break; }
       ++oc;
       tc_fence_after_sync();
       const float inv_l = 1.f / l;
-      const long long tok = static_cast<long long>(b) * p.S + qb * kFaBM + row;
-      elem_t* orow = p.o + tok * p.o_pitch + static_cast<long long>(h) * kFaD;
+      const int qrow = tile * kFaBM + row;
+      const bool live = qrow < p.S;
+      elem_t* orow = p.o + (static_cast<long long>(it.b) * p.S + qrow) * p.o_pitch + static_cast<long long>(it.h) * kFaD;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem_o + lane_sel + c * 32, r);
+        tmem_ld_32x32(tm_o + c * 32, r);
         tmem_ld_wait();
+        if (live) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-          uint4 v;
-          v.x = pack_e2(__uint_as_float(r[i + 0]) * inv_l, __uint_as_float(r[i + 1]) * inv_l);
-          v.y = pack_e2(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l);
-          v.z = pack_e2(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l);
-          v.w = pack_e2(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + c * 32 + i) = v;
+          for (int i = 0; i < 32; i += 8) {
+            uint4 v;
+            v.x = pack_e2(__uint_as_float(r[i + 0]) * inv_l, __uint_as_float(r[i + 1]) * inv_l);
+            v.y = pack_e2(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l);
+            v.z = pack_e2(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l);
+            v.w = pack_e2(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l);
+            *reinterpret_cast<uint4*>(orow + c * 32 + i) = v;
+          }
         }
       }
       tc_fence_before_sync();
-      if (p.lse) {
-        p.lse[(static_cast<long long>(b) * p.H + h) * p.S + qb * kFaBM + row] =
+      if (p.lse && live) {
+        p.lse[(static_cast<long long>(it.b) * p.H + it.h) * p.S + qrow] =
             (m_used + log2f(l)) * 0.6931471805599453f;
       }
     }
@@ -333,7 +370,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // a wait was abandoned: give bulk copies that may still be in flight a bounded time to land
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 100000000ull) {
-      if (mbar_try_wait(q_full, 0) && mbar_try_wait(q_full, 1)) break;
     }
   }
   __syncthreads();
@@ -343,8 +379,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-
-
 }  // namespace MSB_ELEM_NS
 }  // namespace msb
 
@@ -352,13 +386,13 @@ using namespace msb;
 using namespace msb::MSB_ELEM_NS;
 
 // q [B,S,H,128], k/v [B,S,Hk,128] with token pitches (elements) q_pitch / k_pitch / v_pitch; o [B,S,H,128] with o_pitch.
-// S must be a multiple of 128.  lse (fp32 [B,H,S]) may be null.
+// lse (fp32 [B,H,S]) may be null.
 MSB_EXPORT int MSB_FN(msb_flash_attn_fwd)(const void* q, const void* k, const void* v, void* o, float* lse, int B, int S,
                                   int H, int Hk, int D, long long q_pitch, long long k_pitch, long long v_pitch,
                                   long long o_pitch,
                                   int causal, float scale, void* stream_) {
-  if (D != kFaD || S % 128 != 0 || S <= 0 || H % Hk != 0 || B <= 0) {
-    set_last_error("flash_attn_fwd: needs head_dim 128, S a multiple of 128 and H a multiple of Hk "
+  if (D != kFaD || S % 128 != 0 || S <= 0 || Hk <= 0 || H % Hk != 0 || B <= 0) {
+    set_last_error("flash_attn_fwd: needs head_dim 128 and H a multiple of Hk "
                    "(got D=%d S=%d H=%d Hk=%d)", D, S, H, Hk);
     return kBadArg;
   }
@@ -388,7 +422,7 @@ MSB_EXPORT int MSB_FN(msb_flash_attn_fwd)(const void* q, const void* k, const vo
   p.causal = causal;
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const int total = B * H * (S / 128);
+  const int total = B * H * ((S + 255) / 256);
   const int grid = total < sm_count() ? total : sm_count();
   flash_fwd_kernel<<<grid, kFaThreads, FaSmem::kBytes, static_cast<cudaStream_t>(stream_)>>>(tq, tk, tv, p);
   MSB_CUDA_CHECK(cudaGetLastError());

@@ -152,6 +152,28 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// ---- the same, issued by a whole converged warp: one elected lane's instruction takes effect.  The operands of a tcgen05
+// instruction live in uniform registers.  A warp that runs the issuing code together, on values that are the same in all
+// lanes, keeps descriptors there; code under `if (lane == 0)` moves every descriptor over for each instruction, about 100
+// cycles a piece, which a 128 x 128 x 16 product (64 cycles) cannot hide.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(e));
+  return e;
+}
+// Index of this thread's warp in the block, known to the compiler to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+// mbar_wait by all lanes, with one answer for all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const AbortCtx& ab) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, ab));
+}
+
 // Arrive on `bar` once every tcgen05 op issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
