@@ -15,8 +15,6 @@
 namespace msb {
 namespace MSB_ELEM_NS {
 
-constexpr int kNormThreads = 256;
-
 struct alignas(16) bf16x8 {
   elem2_t v[4];
 };
@@ -37,120 +35,271 @@ __device__ __forceinline__ void store8(elem_t* p, const float (&f)[8]) {
   *reinterpret_cast<bf16x8*>(p) = raw;
 }
 
-template <int THREADS>
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  v = warp_sum(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  float t = (lane < THREADS / 32) ? red[lane] : 0.f;
-  t = warp_sum(t);
-  return t;
+// ------------------------------------------------------------------------------------ norms: threads and rows
+// A row of H elements is H / 8 vectors of 16 bytes.  T threads (a multiple of 32) share a row, V vectors each, and a block
+// holds R such groups, each with a row of its own.  The bound is HBM; what costs time beside it is a row's chain of load,
+// reduction and store, so an SM needs many rows in flight and no thread without a vector.  One row per block of 256
+// threads, as before, idled three quarters of the second round of vectors at H = 2560 and held two rows per SM in the
+// backward kernels, whose loads of the residual gradient moreover waited for the reduction.  Measured, bf16: RMSNorm
+// backward of 4096 x 4096 with residual 52 -> 41 us, LayerNorm backward of 8191 x 2560 68 -> 44 us, forward 35 -> 34 us.
+// A forward kernel that prefetches the next row measured no better than one block per row.
+struct NormShape {
+  int T, R, V;
+};
+constexpr int kNormMaxV = 4;
+constexpr int kNormMaxThreads = 512;      // H = 16384
+constexpr int kNormBwdPerSm = 4;          // most blocks per SM of a backward kernel
+
+// Of the shapes with at most max_v vectors per thread the one with the fewest idle slots, the most vectors per thread
+// among those.
+static inline NormShape norm_shape(int H, int max_v) {
+  const int vecs = H / 8;
+  NormShape best = {0, 1, 0};
+  int waste = 1 << 30;
+  for (int v = max_v; v >= 1; --v) {
+    const int t = (vecs + 32 * v - 1) / (32 * v) * 32;
+    if (t <= kNormMaxThreads && t * v - vecs < waste) {
+      waste = t * v - vecs;
+      best.T = t;
+      best.V = v;
+    }
+  }
+  return best;
 }
+// Forward: a warp per row needs no barrier, eight of them make a block; longer rows have the block to themselves.
+static inline NormShape norm_fwd_shape(int H) {
+  NormShape n = norm_shape(H, H <= 16 * kNormMaxThreads ? 2 : kNormMaxV);
+  if (n.T == 32) n.R = 8;
+  return n;
+}
+// Backward: the accumulators of the weight gradients take 8 registers per vector, so two vectors per thread as far as
+// 512 threads reach, and groups of a block share one row of partial sums.
+static inline NormShape norm_bwd_shape(int H) {
+  NormShape n = norm_shape(H, H <= 16 * kNormMaxThreads ? 2 : kNormMaxV);
+  n.R = n.T >= 256 ? 1 : 256 / n.T;
+  return n;
+}
+
+// Reductions over the T threads of a row.  MULTI: several groups per block, each with a named barrier of its own (1 +
+// group); otherwise the group is one warp or the whole block.
+template <bool MULTI>
+struct NormGroup {
+  int T, tid, group, warps, buf;
+  float2* red;                            // [2][16] of this group
+  __device__ __forceinline__ NormGroup(int T_, float2* smem) : T(T_), buf(0) {
+    group = threadIdx.x / T_;
+    tid = threadIdx.x - group * T_;
+    warps = T_ >> 5;
+    red = smem + (MULTI ? group * 32 : 0);
+  }
+  // At most four groups are wider than a warp (T >= 64).  Barrier numbers are constants: a number in a register makes the
+  // compiler reserve all sixteen barriers for every block.
+  __device__ __forceinline__ void barrier() {
+    if (!MULTI) { __syncthreads(); return; }
+    if (group == 0) asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
+    else if (group == 1) asm volatile("bar.sync 2, %0;" ::"r"(T) : "memory");
+    else if (group == 2) asm volatile("bar.sync 3, %0;" ::"r"(T) : "memory");
+    else asm volatile("bar.sync 4, %0;" ::"r"(T) : "memory");
+  }
+  // Sums of a and b over the group, in every thread.  The scratch alternates between two halves: a warp can be at most one
+  // sum ahead of the others of its group.
+  __device__ __forceinline__ float2 sum2(float a, float b) {
+    a = warp_sum(a);
+    b = warp_sum(b);
+    if (warps == 1) return make_float2(a, b);
+    const int lane = tid & 31;
+    float2* half = red + buf * 16;
+    buf ^= 1;
+    if (lane == 0) half[tid >> 5] = make_float2(a, b);
+    barrier();
+    const float2 t = lane < warps ? half[lane] : make_float2(0.f, 0.f);
+    return make_float2(warp_sum(t.x), warp_sum(t.y));
+  }
+  __device__ __forceinline__ float sum(float a) {
+    a = warp_sum(a);
+    if (warps == 1) return a;
+    const int lane = tid & 31;
+    float2* half = red + buf * 16;
+    buf ^= 1;
+    if (lane == 0) half[tid >> 5].x = a;
+    barrier();
+    return warp_sum(lane < warps ? half[lane].x : 0.f);
+  }
+};
+constexpr int kNormRed = 32, kNormRedMulti = 8 * 32;    // float2 scratch of a block (8 groups at most)
+
+__device__ __forceinline__ void unpack8(const bf16x8& raw, float (&f)[8]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = e2_to_f2(raw.v[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ bf16x8 load_raw(const elem_t* p) { return *reinterpret_cast<const bf16x8*>(p); }
 
 // ------------------------------------------------------------------------------------ RMSNorm
 // y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream to `xsum`.
-// H must be a multiple of 8 and <= kNormThreads*8*kMaxIter.
-constexpr int kMaxIter = 8;  // H up to 16384
-
-template <int ITER>
-__global__ void __launch_bounds__(kNormThreads)
+// H must be a multiple of 8 and at most 8 * kNormMaxV * kNormMaxThreads.
+template <int V>
+__global__ void __launch_bounds__(kNormMaxThreads)
 rmsnorm_fwd_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ res,
                    const elem_t* __restrict__ w, elem_t* __restrict__ y,
-                   elem_t* __restrict__ xsum, float* __restrict__ rstd_out, int H, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const elem_t* xr = x + row * H;
-  float v[ITER][8];
-  float ss = 0.f;
+                   elem_t* __restrict__ xsum, float* __restrict__ rstd_out, long long rows, int H, float eps, int T, int R) {
+  __shared__ float2 red[kNormRed];
+  NormGroup<false> g(T, red);
+  const long long row = blockIdx.x * static_cast<long long>(R) + g.group;
+  if (row >= rows) return;
+  float v[V][8];
+  {
+    bf16x8 rx[V], rr[V];
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-    if (c < H) {
-      load8(xr + c, v[it]);
-      if (res) {
-        float r[8];
-        load8(res + row * H + c, r);
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
+        rx[it] = load_raw(x + row * H + c);
+        if (res) rr[it] = load_raw(res + row * H + c);
+      }
+    }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[it][j] += r[j];
-        if (xsum) {
-          // round once so that the normalised value matches what the backward pass re-reads
-          store8(xsum + row * H + c, v[it]);
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
+        unpack8(rx[it], v[it]);
+        if (res) {
+          float r[8];
+          unpack8(rr[it], r);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[it][j] = e_to_f(f_to_e(v[it][j]));
+          for (int j = 0; j < 8; ++j) v[it][j] += r[j];
+          if (xsum) {
+            // round once so that the normalised value matches what the backward pass re-reads
+            store8(xsum + row * H + c, v[it]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[it][j] = e_to_f(f_to_e(v[it][j]));
+          }
         }
       }
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int it = 0; it < V; ++it) {
+    if ((it * T + g.tid) * 8 < H) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += v[it][j] * v[it][j];
     }
   }
-  ss = block_sum<kNormThreads>(ss, red);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
+  const float rstd = rsqrtf(g.sum(ss) / H + eps);
+  if (g.tid == 0 && rstd_out) rstd_out[row] = rstd;
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
+  for (int it = 0; it < V; ++it) {
+    const int c = (it * T + g.tid) * 8;
     if (c < H) {
-      float g[8], o[8];
-      load8(w + c, g);
+      float gm[8], o[8];
+      load8(w + c, gm);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = v[it][j] * rstd * g[j];
+      for (int j = 0; j < 8; ++j) o[j] = v[it][j] * rstd * gm[j];
       store8(y + row * H + c, o);
     }
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres_in) ; dw = sum_rows dy * xhat.
-// Persistent over rows; per-CTA partial dw kept in registers.  Two-stage reduction (ATOMIC = false): CTA b stores
-// its partial as row b of dw_acc[gridDim.x][H] and reduce_partials_kernel sums the rows in a fixed order
-// (deterministic).  ATOMIC = true adds into a single dw_acc[H] instead (the allocation-free entry point, whose
-// scratch is one row).
-template <int ITER, bool ATOMIC>
-__global__ void __launch_bounds__(kNormThreads)
-rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x,
-                   const elem_t* __restrict__ w, const float* __restrict__ rstd,
-                   const elem_t* __restrict__ dres, elem_t* __restrict__ dx,
-                   float* __restrict__ dw_acc, int rows, int H) {
-  __shared__ float red[32];
-  float wreg[ITER][8], dwreg[ITER][8];
+// Adds the groups' partial sums of a block (registers `mine`, element c of the row at (it * T + tid) * 8) in group order
+// through shared memory and stores the total as row blockIdx.x of dst[gridDim.x][H].
+template <int V>
+__device__ __forceinline__ void store_partials(const float (&mine)[V][8], float* dst, float* acc, const NormGroup<true>& g,
+                                               int R, int H) {
+  dst += static_cast<long long>(blockIdx.x) * H;
+#pragma unroll 1
+  for (int k = 0; k < R; ++k) {
+    if (g.group == k) {
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dwreg[it][j] = 0.f;
-    if (c < H) load8(w + c, wreg[it]);
-  }
-  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float rs = rstd[row];
-    float g[ITER][8], xh[ITER][8];
-    float dot = 0.f;
-#pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      const int c = (it * kNormThreads + threadIdx.x) * 8;
-      if (c < H) {
-        load8(dy + row * H + c, g[it]);
-        load8(x + row * H + c, xh[it]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[it][j] *= rs;
-          dwreg[it][j] += g[it][j] * xh[it][j];
-          g[it][j] *= wreg[it][j];
-          dot += g[it][j] * xh[it][j];
+      for (int it = 0; it < V; ++it) {
+        const int c = (it * g.T + g.tid) * 8;
+        if (c < H) {
+          float4 lo = make_float4(mine[it][0], mine[it][1], mine[it][2], mine[it][3]);
+          float4 hi = make_float4(mine[it][4], mine[it][5], mine[it][6], mine[it][7]);
+          if (k > 0) {
+            const float4 a = *reinterpret_cast<const float4*>(acc + c), b = *reinterpret_cast<const float4*>(acc + c + 4);
+            lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+            hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+          }
+          float* out = k == R - 1 ? dst : acc;
+          *reinterpret_cast<float4*>(out + c) = lo;
+          *reinterpret_cast<float4*>(out + c + 4) = hi;
         }
       }
     }
-    dot = block_sum<kNormThreads>(dot, red) / H;
+    if (R > 1) __syncthreads();
+  }
+}
+
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres_in) ; dw = sum_rows dy * xhat.
+// Persistent over rows; per-group partial dw kept in registers.  Two-stage reduction (ATOMIC = false): CTA b stores the sum
+// of its groups as row b of dw_acc[gridDim.x][H] and reduce_partials_kernel sums the rows in a fixed order
+// (deterministic).  ATOMIC = true adds into a single dw_acc[H] instead (the allocation-free entry point, whose
+// scratch is one row).  All loads of a row, the residual gradient's too, are issued before its reduction.
+template <int V, bool ATOMIC>
+__global__ void __maxnreg__(V <= 2 ? 64 : 128)
+rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x,
+                   const elem_t* __restrict__ w, const float* __restrict__ rstd,
+                   const elem_t* __restrict__ dres, elem_t* __restrict__ dx,
+                   float* __restrict__ dw_acc, long long rows, int H, int T, int R) {
+  extern __shared__ float part[];          // [H] when R > 1
+  __shared__ float2 red[kNormRedMulti];
+  NormGroup<true> g(T, red);
+  float dwreg[V][8];
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      const int c = (it * kNormThreads + threadIdx.x) * 8;
+  for (int it = 0; it < V; ++it)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dwreg[it][j] = 0.f;
+#pragma unroll 1
+  for (long long row = blockIdx.x * static_cast<long long>(R) + g.group; row < rows;
+       row += static_cast<long long>(gridDim.x) * R) {
+    const float rs = rstd[row];
+    const elem_t* wp = w;                  // opaque: w comes from the L1 cache instead of filling registers
+    asm volatile("" : "+l"(wp));
+    bf16x8 rg[V], rx[V], rd[V];            // kept as loaded and unpacked twice: half the registers of fp32 values
+    float dot = 0.f;
+#pragma unroll
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
       if (c < H) {
-        float o[8];
+        rg[it] = load_raw(dy + row * H + c);
+        rx[it] = load_raw(x + row * H + c);
+        if (dres) rd[it] = load_raw(dres + row * H + c);
+      }
+    }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (g[it][j] - xh[it][j] * dot);
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
+        float wv[8], gv[8], xh[8];
+        load8(wp + c, wv);
+        unpack8(rg[it], gv);
+        unpack8(rx[it], xh);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          xh[j] *= rs;
+          dwreg[it][j] += gv[j] * xh[j];
+          dot += (gv[j] * wv[j]) * xh[j];
+        }
+      }
+    }
+    dot = g.sum(dot) / H;
+#pragma unroll
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
+        float wv[8], gv[8], xh[8], o[8];
+        load8(wp + c, wv);
+        unpack8(rg[it], gv);
+        unpack8(rx[it], xh);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = rs * (gv[j] * wv[j] - xh[j] * rs * dot);
         if (dres) {
           float r[8];
-          load8(dres + row * H + c, r);
+          unpack8(rd[it], r);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += r[j];
         }
@@ -158,70 +307,86 @@ rmsnorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x,
       }
     }
   }
+  if (ATOMIC) {
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-    if (c < H) {
-      if (ATOMIC) {
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) atomicAdd(dw_acc + c + j, dwreg[it][j]);
-      } else {
-        float* dst = dw_acc + static_cast<long long>(blockIdx.x) * H + c;
-        *reinterpret_cast<float4*>(dst) = make_float4(dwreg[it][0], dwreg[it][1], dwreg[it][2], dwreg[it][3]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(dwreg[it][4], dwreg[it][5], dwreg[it][6], dwreg[it][7]);
       }
     }
+  } else {
+    store_partials<V>(dwreg, dw_acc, part, g, R, H);
   }
 }
 
 // Second stage of the weight-gradient reduction: out[c] (+)= sum_b partial[b][c] for b = 0..parts-1, rows visited
 // in a fixed order.  Block = 32 columns x 8 row lanes; lane r sums rows r, r+8, ... and the 8 lanes are combined
-// through shared memory, always in the same order.
+// through shared memory, always in the same order.  blockIdx.y chooses between two such reductions (dw, db).
+struct PartialsOut {
+  const float* partial;
+  elem_t* out_bf16;
+  float* out_f32;
+};
 __global__ void __launch_bounds__(256)
-reduce_partials_kernel(const float* __restrict__ partial, int parts, int H, elem_t* __restrict__ out_bf16,
-                       float* __restrict__ out_f32, int accumulate) {
+reduce_partials_kernel(const PartialsOut first, const PartialsOut second, int parts, int H, int accumulate) {
   __shared__ float sm[8][33];
+  const PartialsOut o = blockIdx.y == 0 ? first : second;
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float s = 0.f;
-  if (c < H)
-    for (int b = ry; b < parts; b += 8) s += partial[static_cast<long long>(b) * H + c];
+  if (c < H) {
+#pragma unroll 8
+    for (int b = ry; b < parts; b += 8) s += o.partial[static_cast<long long>(b) * H + c];
+  }
   sm[ry][cx] = s;
   __syncthreads();
   if (ry == 0 && c < H) {
     float v = sm[0][cx];
 #pragma unroll
     for (int r = 1; r < 8; ++r) v += sm[r][cx];
-    if (out_f32) out_f32[c] = accumulate ? out_f32[c] + v : v;
-    if (out_bf16) out_bf16[c] = f_to_e(accumulate ? e_to_f(out_bf16[c]) + v : v);
+    if (o.out_f32) o.out_f32[c] = accumulate ? o.out_f32[c] + v : v;
+    if (o.out_bf16) o.out_bf16[c] = f_to_e(accumulate ? e_to_f(o.out_bf16[c]) + v : v);
   }
 }
 
 // ------------------------------------------------------------------------------------ LayerNorm
-template <int ITER>
-__global__ void __launch_bounds__(kNormThreads)
+template <int V>
+__global__ void __launch_bounds__(kNormMaxThreads)
 layernorm_fwd_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ w,
                      const elem_t* __restrict__ b, elem_t* __restrict__ y,
-                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int H, float eps) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  float v[ITER][8];
+                     float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int H, float eps, int T,
+                     int R) {
+  __shared__ float2 red[kNormRed];
+  NormGroup<false> g(T, red);
+  const long long row = blockIdx.x * static_cast<long long>(R) + g.group;
+  if (row >= rows) return;
+  float v[V][8];
+  {
+    bf16x8 rx[V];
+#pragma unroll
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) rx[it] = load_raw(x + row * H + c);
+    }
+#pragma unroll
+    for (int it = 0; it < V; ++it)
+      if ((it * T + g.tid) * 8 < H) unpack8(rx[it], v[it]);
+  }
   float s = 0.f;
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-    if (c < H) {
-      load8(x + row * H + c, v[it]);
+  for (int it = 0; it < V; ++it) {
+    if ((it * T + g.tid) * 8 < H) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += v[it][j];
     }
   }
-  const float mean = block_sum<kNormThreads>(s, red) / H;
+  const float mean = g.sum(s) / H;
   float ss = 0.f;
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-    if (c < H) {
+  for (int it = 0; it < V; ++it) {
+    if ((it * T + g.tid) * 8 < H) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float d = v[it][j] - mean;
@@ -229,89 +394,94 @@ layernorm_fwd_kernel(const elem_t* __restrict__ x, const elem_t* __restrict__ w,
       }
     }
   }
-  const float rstd = rsqrtf(block_sum<kNormThreads>(ss, red) / H + eps);
-  if (threadIdx.x == 0) {
+  const float rstd = rsqrtf(g.sum(ss) / H + eps);
+  if (g.tid == 0) {
     if (mean_out) mean_out[row] = mean;
     if (rstd_out) rstd_out[row] = rstd;
   }
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
+  for (int it = 0; it < V; ++it) {
+    const int c = (it * T + g.tid) * 8;
     if (c < H) {
-      float g[8], bb[8], o[8];
-      load8(w + c, g);
+      float gm[8], bb[8], o[8];
+      load8(w + c, gm);
       if (b) load8(b + c, bb);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = (v[it][j] - mean) * rstd * g[j] + (b ? bb[j] : 0.f);
+      for (int j = 0; j < 8; ++j) o[j] = (v[it][j] - mean) * rstd * gm[j] + (b ? bb[j] : 0.f);
       store8(y + row * H + c, o);
     }
   }
 }
 
-template <int ITER>
-__global__ void __launch_bounds__(kNormThreads)
+template <int V>
+__global__ void __maxnreg__(V <= 2 ? 80 : 128)
 layernorm_bwd_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x,
                      const elem_t* __restrict__ w, const float* __restrict__ mean,
                      const float* __restrict__ rstd, elem_t* __restrict__ dx, float* __restrict__ dw_acc,
-                     float* __restrict__ db_acc, int rows, int H) {
-  __shared__ float red[32];
-  float wreg[ITER][8], dwreg[ITER][8], dbreg[ITER][8];
+                     float* __restrict__ db_acc, long long rows, int H, int T, int R) {
+  extern __shared__ float part[];          // [H] when R > 1
+  __shared__ float2 red[kNormRedMulti];
+  NormGroup<true> g(T, red);
+  float dwreg[V][8], dbreg[V][8];
 #pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
+  for (int it = 0; it < V; ++it)
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwreg[it][j] = dbreg[it][j] = 0.f;
-    if (c < H) load8(w + c, wreg[it]);
-  }
-  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+#pragma unroll 1
+  for (long long row = blockIdx.x * static_cast<long long>(R) + g.group; row < rows;
+       row += static_cast<long long>(gridDim.x) * R) {
     const float mu = mean[row], rs = rstd[row];
-    float g[ITER][8], xh[ITER][8];
+    const elem_t* wp = w;
+    asm volatile("" : "+l"(wp));
+    bf16x8 rg[V], rx[V];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      const int c = (it * kNormThreads + threadIdx.x) * 8;
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
       if (c < H) {
-        load8(dy + row * H + c, g[it]);
-        load8(x + row * H + c, xh[it]);
+        rg[it] = load_raw(dy + row * H + c);
+        rx[it] = load_raw(x + row * H + c);
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
+      if (c < H) {
+        float wv[8], gv[8], xh[8];
+        load8(wp + c, wv);
+        unpack8(rg[it], gv);
+        unpack8(rx[it], xh);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[it][j] = (xh[it][j] - mu) * rs;
-          dwreg[it][j] += g[it][j] * xh[it][j];
-          dbreg[it][j] += g[it][j];
-          g[it][j] *= wreg[it][j];
-          s1 += g[it][j];
-          s2 += g[it][j] * xh[it][j];
+          xh[j] = (xh[j] - mu) * rs;
+          dwreg[it][j] += gv[j] * xh[j];
+          dbreg[it][j] += gv[j];
+          gv[j] *= wv[j];
+          s1 += gv[j];
+          s2 += gv[j] * xh[j];
         }
       }
     }
-    s1 = block_sum<kNormThreads>(s1, red) / H;
-    s2 = block_sum<kNormThreads>(s2, red) / H;
+    const float2 t = g.sum2(s1, s2);
+    s1 = t.x / H;
+    s2 = t.y / H;
 #pragma unroll
-    for (int it = 0; it < ITER; ++it) {
-      const int c = (it * kNormThreads + threadIdx.x) * 8;
+    for (int it = 0; it < V; ++it) {
+      const int c = (it * T + g.tid) * 8;
       if (c < H) {
-        float o[8];
+        float wv[8], gv[8], xh[8], o[8];
+        load8(wp + c, wv);
+        unpack8(rg[it], gv);
+        unpack8(rx[it], xh);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (g[it][j] - s1 - xh[it][j] * s2);
+        for (int j = 0; j < 8; ++j) o[j] = rs * (gv[j] * wv[j] - s1 - (xh[j] - mu) * rs * s2);
         store8(dx + row * H + c, o);
       }
     }
   }
   // two-stage reduction: this CTA's partial sums are row blockIdx.x of dw_acc / db_acc ([gridDim.x][H] each)
-#pragma unroll
-  for (int it = 0; it < ITER; ++it) {
-    const int c = (it * kNormThreads + threadIdx.x) * 8;
-    if (c < H) {
-      float* dw = dw_acc + static_cast<long long>(blockIdx.x) * H + c;
-      *reinterpret_cast<float4*>(dw) = make_float4(dwreg[it][0], dwreg[it][1], dwreg[it][2], dwreg[it][3]);
-      *reinterpret_cast<float4*>(dw + 4) = make_float4(dwreg[it][4], dwreg[it][5], dwreg[it][6], dwreg[it][7]);
-      if (db_acc) {
-        float* db = db_acc + static_cast<long long>(blockIdx.x) * H + c;
-        *reinterpret_cast<float4*>(db) = make_float4(dbreg[it][0], dbreg[it][1], dbreg[it][2], dbreg[it][3]);
-        *reinterpret_cast<float4*>(db + 4) = make_float4(dbreg[it][4], dbreg[it][5], dbreg[it][6], dbreg[it][7]);
-      }
-    }
-  }
+  store_partials<V>(dwreg, dw_acc, part, g, R, H);
+  if (db_acc) store_partials<V>(dbreg, db_acc, part, g, R, H);
 }
 
 // fp32 accumulator -> bf16 parameter gradient (optionally accumulating into an existing bf16/fp32 grad)
@@ -447,31 +617,43 @@ static inline int ew_grid(long long work_items, int threads) {
 using namespace msb;
 using namespace msb::MSB_ELEM_NS;
 
-#define MSB_ITER_DISPATCH(H, CALL)                                           \
-  do {                                                                       \
-    const int _it = ((H) / 8 + kNormThreads - 1) / kNormThreads;             \
-    if (_it <= 1) { CALL(1); } else if (_it <= 2) { CALL(2); }               \
-    else if (_it <= 4) { CALL(4); } else { CALL(8); }                        \
+#define MSB_NORM_DISPATCH(V, CALL) \
+  do {                             \
+    if ((V) == 1) { CALL(1); }     \
+    else if ((V) == 2) { CALL(2); } \
+    else if ((V) == 3) { CALL(3); } \
+    else { CALL(4); }              \
   } while (0)
 
 static int check_h(const char* what, int H) {
-  if (H <= 0 || (H % 8) != 0 || H > kNormThreads * 8 * kMaxIter) {
+  if (H <= 0 || (H % 8) != 0 || H > 8 * kNormMaxV * kNormMaxThreads) {
     set_last_error("%s: hidden size %d must be a positive multiple of 8 and <= %d", what, H,
-                   kNormThreads * 8 * kMaxIter);
+                   8 * kNormMaxV * kNormMaxThreads);
     return kBadArg;
   }
   return kOk;
 }
 
+// Blocks of a backward kernel: as many as are resident (`threads` per SM at the kernel's registers), fewer where the rows
+// run out.  The scratch holds a partial row for each.
+static int norm_bwd_grid(long long rows, const NormShape& n, int threads) {
+  int per = threads / (n.T * n.R);
+  per = per < 1 ? 1 : (per > kNormBwdPerSm ? kNormBwdPerSm : per);
+  const long long need = (rows + n.R - 1) / n.R, cap = (long long)per * sm_count();
+  return (int)(need < cap ? need : cap);
+}
+constexpr int kRmsBwdThreads = 1024, kLnBwdThreads = 768;
+
 MSB_EXPORT int MSB_FN(msb_rmsnorm_fwd)(const void* x, const void* res, const void* w, void* y, void* xsum, float* rstd,
                                long long rows, int H, float eps, void* stream) {
   if (int rc = check_h("rmsnorm_fwd", H)) return rc;
   if (rows <= 0) return kOk;
-#define CALL(I)                                                                                          \
-  rmsnorm_fwd_kernel<I><<<(unsigned)rows, kNormThreads, 0, (cudaStream_t)stream>>>(                      \
+  const NormShape n = norm_fwd_shape(H);
+#define CALL(V_)                                                                                         \
+  rmsnorm_fwd_kernel<V_><<<(unsigned)((rows + n.R - 1) / n.R), n.T * n.R, 0, (cudaStream_t)stream>>>(      \
       (const elem_t*)x, (const elem_t*)res, (const elem_t*)w, (elem_t*)y,    \
-      (elem_t*)xsum, rstd, H, eps)
-  MSB_ITER_DISPATCH(H, CALL);
+      (elem_t*)xsum, rstd, rows, H, eps, n.T, n.R)
+  MSB_NORM_DISPATCH(n.V, CALL);
 #undef CALL
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -481,7 +663,7 @@ MSB_EXPORT int MSB_FN(msb_rmsnorm_fwd)(const void* x, const void* res, const voi
 // Floats of scratch the norm backward launchers need for hidden size H: one partial row per CTA.
 #ifndef MSB_ELEM_FP16
 MSB_EXPORT long long msb_norm_bwd_scratch_elems(int H, int with_bias) {
-  return 2LL * sm_count() * H * (with_bias ? 2 : 1);
+  return (long long)kNormBwdPerSm * sm_count() * H * (with_bias ? 2 : 1);
 }
 #endif
 
@@ -493,17 +675,18 @@ MSB_EXPORT int MSB_FN(msb_rmsnorm_bwd)(const void* dy, const void* x, const void
   cudaStream_t stream = (cudaStream_t)stream_;
   int grid = 0;
   if (rows > 0) {
-    grid = (int)(rows < 2LL * sm_count() ? rows : 2LL * sm_count());
-#define CALL(I)                                                                                      \
-  rmsnorm_bwd_kernel<I, false><<<grid, kNormThreads, 0, stream>>>(                                   \
+    const NormShape n = norm_bwd_shape(H);
+    grid = norm_bwd_grid(rows, n, kRmsBwdThreads);
+#define CALL(V_)                                                                                     \
+  rmsnorm_bwd_kernel<V_, false><<<grid, n.T * n.R, n.R > 1 ? H * 4 : 0, stream>>>(                    \
       (const elem_t*)dy, (const elem_t*)x, (const elem_t*)w, rstd,              \
-      (const elem_t*)dres, (elem_t*)dx, dw_acc, (int)rows, H)
-    MSB_ITER_DISPATCH(H, CALL);
+      (const elem_t*)dres, (elem_t*)dx, dw_acc, rows, H, n.T, n.R)
+    MSB_NORM_DISPATCH(n.V, CALL);
 #undef CALL
   }
   if (dw_out) {
-    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(dw_acc, grid, H, dw_fp32 ? nullptr : (elem_t*)dw_out,
-                                                             dw_fp32 ? (float*)dw_out : nullptr, accumulate);
+    const PartialsOut dw = {dw_acc, dw_fp32 ? nullptr : (elem_t*)dw_out, dw_fp32 ? (float*)dw_out : nullptr};
+    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(dw, dw, grid, H, accumulate);
   }
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -513,11 +696,11 @@ MSB_EXPORT int MSB_FN(msb_layernorm_fwd)(const void* x, const void* w, const voi
                                  long long rows, int H, float eps, void* stream) {
   if (int rc = check_h("layernorm_fwd", H)) return rc;
   if (rows <= 0) return kOk;
-#define CALL(I)                                                                                       \
-  layernorm_fwd_kernel<I><<<(unsigned)rows, kNormThreads, 0, (cudaStream_t)stream>>>(                 \
-      (const elem_t*)x, (const elem_t*)w, (const elem_t*)b, (elem_t*)y,   \
-      mean, rstd, H, eps)
-  MSB_ITER_DISPATCH(H, CALL);
+  const NormShape n = norm_fwd_shape(H);
+#define CALL(V_)                                                                                         \
+  layernorm_fwd_kernel<V_><<<(unsigned)((rows + n.R - 1) / n.R), n.T * n.R, 0, (cudaStream_t)stream>>>(    \
+      (const elem_t*)x, (const elem_t*)w, (const elem_t*)b, (elem_t*)y, mean, rstd, rows, H, eps, n.T, n.R)
+  MSB_NORM_DISPATCH(n.V, CALL);
 #undef CALL
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -530,23 +713,23 @@ MSB_EXPORT int MSB_FN(msb_layernorm_bwd)(const void* dy, const void* x, const vo
   if (int rc = check_h("layernorm_bwd", H)) return rc;
   cudaStream_t stream = (cudaStream_t)stream_;
   int grid = 0;
-  float* db_part = acc + 2LL * sm_count() * H;
+  float* db_part = acc + (long long)kNormBwdPerSm * sm_count() * H;
   if (rows > 0) {
-    grid = (int)(rows < 2LL * sm_count() ? rows : 2LL * sm_count());
-#define CALL(I)                                                                                   \
-  layernorm_bwd_kernel<I><<<grid, kNormThreads, 0, stream>>>(                                     \
+    const NormShape n = norm_bwd_shape(H);
+    grid = norm_bwd_grid(rows, n, kLnBwdThreads);
+#define CALL(V_)                                                                                  \
+  layernorm_bwd_kernel<V_><<<grid, n.T * n.R, n.R > 1 ? H * 4 : 0, stream>>>(                      \
       (const elem_t*)dy, (const elem_t*)x, (const elem_t*)w, mean, rstd,     \
-      (elem_t*)dx, acc, db_out ? db_part : nullptr, (int)rows, H)
-    MSB_ITER_DISPATCH(H, CALL);
+      (elem_t*)dx, acc, db_out ? db_part : nullptr, rows, H, n.T, n.R)
+    MSB_NORM_DISPATCH(n.V, CALL);
 #undef CALL
   }
-  if (dw_out)
-    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(acc, grid, H, out_fp32 ? nullptr : (elem_t*)dw_out,
-                                                             out_fp32 ? (float*)dw_out : nullptr, accumulate);
-  if (db_out)
-    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(db_part, grid, H,
-                                                             out_fp32 ? nullptr : (elem_t*)db_out,
-                                                             out_fp32 ? (float*)db_out : nullptr, accumulate);
+  const PartialsOut dw = {acc, out_fp32 ? nullptr : (elem_t*)dw_out, out_fp32 ? (float*)dw_out : nullptr};
+  const PartialsOut db = {db_part, out_fp32 ? nullptr : (elem_t*)db_out, out_fp32 ? (float*)db_out : nullptr};
+  if (dw_out && db_out)
+    reduce_partials_kernel<<<dim3((H + 31) / 32, 2), 256, 0, stream>>>(dw, db, grid, H, accumulate);
+  else if (dw_out || db_out)
+    reduce_partials_kernel<<<(H + 31) / 32, 256, 0, stream>>>(dw_out ? dw : db, db, grid, H, accumulate);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
@@ -642,12 +825,13 @@ MSB_EXPORT int msb_rmsnorm_bwd_static(const void* dy, const void* x, const void*
   cudaStream_t stream = (cudaStream_t)stream_;
   MSB_CUDA_CHECK(cudaMemsetAsync(acc, 0, sizeof(float) * H, stream));
   if (rows > 0) {
-    const int grid = (int)(rows < 2LL * sm_count() ? rows : 2LL * sm_count());
-#define CALL(I)                                                                                      \
-  rmsnorm_bwd_kernel<I, true><<<grid, kNormThreads, 0, stream>>>(                                    \
+    const NormShape n = norm_bwd_shape(H);
+    const int grid = norm_bwd_grid(rows, n, kRmsBwdThreads);
+#define CALL(V_)                                                                                     \
+  rmsnorm_bwd_kernel<V_, true><<<grid, n.T * n.R, 0, stream>>>(                                       \
       (const elem_t*)dy, (const elem_t*)x, (const elem_t*)w, rstd,              \
-      (const elem_t*)dres, (elem_t*)dx, acc, (int)rows, H)
-    MSB_ITER_DISPATCH(H, CALL);
+      (const elem_t*)dres, (elem_t*)dx, acc, rows, H, n.T, n.R)
+    MSB_NORM_DISPATCH(n.V, CALL);
 #undef CALL
   }
   if (dw_out) {

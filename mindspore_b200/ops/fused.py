@@ -145,6 +145,7 @@ class _RmsNormFn(torch.autograd.Function):
         ctx.save_for_backward(xsum, w, rstd)
         ctx.w_ref = w
         ctx.has_res = residual is not None
+        ctx.set_materialize_grads(False)          # no zero gradients for the outputs nothing is derived from
         rstd_out = rstd.view_as(rstd)
         ctx.mark_non_differentiable(rstd_out)
         if residual is not None:
@@ -156,6 +157,8 @@ class _RmsNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dxsum, _drstd):
         xsum, w, rstd = ctx.saved_tensors
+        if dy is None:
+            dy = torch.zeros_like(xsum)
         mg = getattr(ctx.w_ref, "main_grad", None)
         dres = dxsum.contiguous() if (ctx.has_res and dxsum is not None) else None
         dx, dw = K.rmsnorm_bwd(dy.contiguous(), xsum, w, rstd, dresidual=dres, dw_out=mg, accumulate=mg is not None)

@@ -69,3 +69,32 @@ def test_cross_entropy_without_a_valid_row(K):
     loss = fused.softmax_cross_entropy(x, torch.full((4,), -100, device=DEV, dtype=torch.int32))
     loss.backward()
     assert float(loss) == 0 and not x.grad.any()
+
+
+# ------------------------------------------------------------------------------------------------ norms
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 248), (700, 256), (5, 1032), (1031, 2560), (2, 5064), (601, 4096),
+                                    (7, 8200), (3, 16384)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_norms_over_the_range_of_widths(K, rows, H, dtype):
+    """A warp per row, groups of a block, whole blocks of every size; fewer rows than SMs and several per CTA."""
+    x, r, dy, ds = (torch.randn(rows, H, device=DEV).to(dtype) for _ in range(4))
+    w, b = ((1 + 0.1 * torch.randn(H, device=DEV)).to(dtype) for _ in range(2))
+    y, rstd, s = K.rmsnorm_fwd(x, w, 1e-5, residual=r)
+    dx, dw = K.rmsnorm_bwd(dy, s, w, rstd, dresidual=ds)
+    acc = torch.ones(H, device=DEV)
+    K.rmsnorm_bwd(dy, s, w, rstd, dw_out=acc, accumulate=True)
+    sd, wd = s.double().requires_grad_(True), w.double().requires_grad_(True)
+    ref = sd * torch.rsqrt(sd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    ref.backward(dy.double())
+    assert torch.equal(s, (x.float() + r.float()).to(dtype))
+    _near(y, ref, 2, dtype)
+    _near(dx, sd.grad + ds.double(), 2, dtype)
+    _near(dw, wd.grad, 2, dtype)
+    _near(acc - 1, wd.grad, 2, dtype)
+    y, mean, rstd = K.layernorm_fwd(x, w, b, 1e-5)
+    dx, dw, db = K.layernorm_bwd(dy, x, w, mean, rstd)
+    xd, wd, bd = (t.double().requires_grad_(True) for t in (x, w, b))
+    ref = torch.nn.functional.layer_norm(xd, (H,), wd, bd, 1e-5)
+    ref.backward(dy.double())
+    for got, exp in ((y, ref), (dx, xd.grad), (dw, wd.grad), (db, bd.grad)):
+        _near(got, exp, 2, dtype)
