@@ -391,7 +391,7 @@ MSB_EXPORT int MSB_FN(msb_flash_attn_fwd)(const void* q, const void* k, const vo
                                   int H, int Hk, int D, long long q_pitch, long long k_pitch, long long v_pitch,
                                   long long o_pitch,
                                   int causal, float scale, void* stream_) {
-  if (D != kFaD || S % 128 != 0 || S <= 0 || Hk <= 0 || H % Hk != 0 || B <= 0) {
+  if (D != kFaD || S <= 0 || Hk <= 0 || H % Hk != 0 || B <= 0) {
     set_last_error("flash_attn_fwd: needs head_dim 128 and H a multiple of Hk "
                    "(got D=%d S=%d H=%d Hk=%d)", D, S, H, Hk);
     return kBadArg;

@@ -41,6 +41,6 @@ def reference_attention(q, k, v, causal=True, scale=None):
 
 def flash_attention(q, k, v, causal=True, scale=None):
     impl = _kernel_impl()
-    if impl and impl.supports(q, k, v):
+    if impl and impl.supports(q, k, v) and (scale is None or scale > 0):      # the kernel's running maximum needs that
         return impl.flash_attention(q, k, v, causal, scale)
     return reference_attention(q, k, v, causal, scale)

@@ -21,14 +21,21 @@ def has_strided_bwd():
     return hasattr(_native.cuda(), "msb_flash_attn_bwd_strided")
 
 
+def _stats_scratch(q):
+    """Two fp32 values per (batch, head, row), rows in whole blocks of 128: what the backward kernels read of the forward
+    pass (-lse * log2 e) and of dO (-scale * <O, dO>)."""
+    B, S, H, _ = q.shape
+    return torch.empty(2 * B * H * ((S + 127) // 128 * 128), dtype=torch.float32, device=q.device)
+
+
 def bwd_into(do, q, k, v, o, lse, causal, scale, dq, dk, dv, grad_pitch):
     """Backward with dq / dk / dv written into caller-provided column blocks (token pitch ``grad_pitch``)."""
     B, S, H, D = q.shape
     Hk = k.shape[2]
     do = do.contiguous()
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
+    stats = _stats_scratch(q)
     rc = K._fn("msb_flash_attn_bwd_strided", q)(
-        _p(q), _p(k), _p(v), _p(o), _p(do), _p(lse), _p(delta), _p(dq), _p(dk), _p(dv), B, S, H, Hk, D,
+        _p(q), _p(k), _p(v), _p(o), _p(do), _p(lse), _p(stats), _p(dq), _p(dk), _p(dv), B, S, H, Hk, D,
         _token_major(q), _token_major(k), _token_major(v), H * D, H * D, grad_pitch, grad_pitch, int(causal),
         float(scale), _stream())
     _native.check(rc, "flash_attn_bwd_strided")
@@ -56,7 +63,8 @@ def supports(q, k, v):
     if not (q.is_cuda and q.dtype in (torch.bfloat16, torch.float16) and k.dtype == q.dtype and v.dtype == q.dtype):
         return False
     B, S, H, D = q.shape
-    return D == 128 and S % 128 == 0 and k.shape[1] == S and H % k.shape[2] == 0 and k.shape[3] == 128
+    return D == 128 and S > 0 and k.shape[:2] == v.shape[:2] == q.shape[:2] and k.shape[2:] == v.shape[2:] \
+        and H % k.shape[2] == 0 and k.shape[3] == 128
 
 
 def fwd(q, k, v, causal, scale):
@@ -82,31 +90,19 @@ def fwd(q, k, v, causal, scale):
 
 
 def bwd(do, q, k, v, o, lse, causal, scale):
-    lib = _native.cuda()
     B, S, H, D = q.shape
     Hk = k.shape[2]
-    if not hasattr(lib, "msb_flash_attn_bwd") or Hk != H:
-        return _bwd_reference(do, q, k, v, causal, scale)
     do = do.contiguous()
     qp, kp = _token_major(q), _token_major(k)
     dq = torch.empty((B, S, H, D), dtype=q.dtype, device=q.device)
     dk = torch.empty((B, S, Hk, D), dtype=q.dtype, device=q.device)
     dv = torch.empty((B, S, Hk, D), dtype=q.dtype, device=q.device)
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-    rc = K._fn("msb_flash_attn_bwd", q)(_p(q), _p(k), _p(v), _p(o), _p(do), _p(lse), _p(delta), _p(dq), _p(dk), _p(dv), B, S, H,
+    stats = _stats_scratch(q)
+    rc = K._fn("msb_flash_attn_bwd", q)(_p(q), _p(k), _p(v), _p(o), _p(do), _p(lse), _p(stats), _p(dq), _p(dk), _p(dv), B, S, H,
                                 Hk, D, qp, kp, _token_major(v), H * D, H * D, int(causal), float(scale), _stream())
     _native.check(rc, "flash_attn_bwd")
     _count(3)
     return dq, dk, dv
-
-
-def _bwd_reference(do, q, k, v, causal, scale):
-    """Recompute-and-differentiate path used where the backward kernel does not apply (e.g. grouped kv heads)."""
-    from .attention import reference_attention
-    with torch.enable_grad():
-        qq, kk, vv = (t.detach().requires_grad_(True) for t in (q, k, v))
-        out = reference_attention(qq, kk, vv, causal, scale)
-        return torch.autograd.grad(out, (qq, kk, vv), do)
 
 
 class _FlashFn(torch.autograd.Function):

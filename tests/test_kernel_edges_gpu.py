@@ -36,6 +36,35 @@ def _status_ok():
     assert _native.device_status() == 0
 
 
+# ------------------------------------------------------------------------------------------------ attention
+@pytest.mark.parametrize("B,S,H,Hk,causal", [(1, 128, 2, 1, True), (2, 384, 4, 2, True), (1, 384, 4, 1, False),
+                                              (1, 640, 40, 40, True), (1, 2176, 12, 3, True), (3, 5, 2, 2, True),
+                                              (2, 100, 2, 1, False), (1, 129, 4, 2, True), (2, 1000, 4, 4, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_flash_attention_grouped_heads_and_odd_tiles(K, B, S, H, Hk, causal, dtype):
+    """One tile, an odd number of query tiles (the second of a pair lies beyond the sequence), more items than SMs,
+    grouped k / v heads, sequences that end inside a tile: forward, log-sum-exp and all gradients."""
+    from mindspore_b200.ops import flash_attn_kernel as FK
+    D = 128
+    q = torch.randn(B, S, H, D, device=DEV).to(dtype)
+    k, v = (torch.randn(B, S, Hk, D, device=DEV).to(dtype) for _ in range(2))
+    do = torch.randn(B, S, H, D, device=DEV).to(dtype)
+    sc = 1 / math.sqrt(D)
+    o, lse, q2, k2, v2 = FK.fwd(q, k, v, causal, sc)
+    dq, dk, dv = FK.bwd(do, q2, k2, v2, o, lse, causal, sc)
+    qf, kf, vf = (t.double().requires_grad_(True) for t in (q, k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", qf, kf.repeat_interleave(H // Hk, 2)) * sc
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), -math.inf)
+    ref = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), vf.repeat_interleave(H // Hk, 2))
+    ref.backward(do.double())
+    _near(o, ref, 4, dtype)                                  # P and O rounded; P's error averages over the keys
+    _near(lse, torch.logsumexp(s, -1), 64, torch.float32)    # exp2 / log2 of the fast unit: 2 ulp each
+    for got, t in ((dq, qf), (dk, kf), (dv, vf)):
+        _near(got, t.grad, 6, dtype)                         # P, dS, O and the result rounded
+    _status_ok()
+
+
 # ------------------------------------------------------------------------------------------------ cross entropy
 @pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (5, 4099), (64, 32000), (9, 50257)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
