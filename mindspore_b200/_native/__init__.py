@@ -58,6 +58,7 @@ _CUDA_SIGNATURES = {
     "msb_layernorm_fwd": (_I, [_P, _P, _P, _P, _P, _P, _L, _I, _F, _P]),
     "msb_layernorm_bwd": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _L, _I, _P]),
     "msb_rope": (_I, [_P, _P, _P, _P, _L, _I, _I, _L, _I, _I, _P]),
+    "msb_rope_to": (_I, [_P, _P, _P, _P, _P, _L, _I, _I, _L, _L, _I, _I, _P]),
     "msb_swiglu_fwd": (_I, [_P, _P, _L, _I, _P]),
     "msb_swiglu_bwd": (_I, [_P, _P, _P, _L, _I, _P]),
     "msb_gelu": (_I, [_P, _P, _P, _P, _L, _I, _I, _P]),

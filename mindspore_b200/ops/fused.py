@@ -268,17 +268,13 @@ class _RopeFn(torch.autograd.Function):
     def forward(ctx, x, cos, sin, heads, head_dim, seq):
         ctx.save_for_backward(cos, sin)
         ctx.meta = (heads, head_dim, seq)
-        out = x.clone()
-        K.rope_(out, cos, sin, heads, head_dim, seq)
-        return out
+        return K.rope(x, cos, sin, heads, head_dim, seq)
 
     @staticmethod
     def backward(ctx, dy):
         cos, sin = ctx.saved_tensors
         heads, head_dim, seq = ctx.meta
-        dx = dy.clone()
-        K.rope_(dx, cos, sin, heads, head_dim, seq, backward=True)
-        return dx, None, None, None, None, None
+        return K.rope(dy.contiguous(), cos, sin, heads, head_dim, seq, backward=True), None, None, None, None, None
 
 
 def rope_tables(seq, head_dim, theta=10000.0, device="cpu"):
@@ -375,29 +371,34 @@ class _QkvRopeAttnFn(torch.autograd.Function):
 
     ``qkv`` [tokens, (H + 2 Hk) * D] is rotated in place (q and k column blocks), the attention kernel reads q, k, v
     as strided views of it, and the backward kernels write dq, dk, dv into the column blocks of one packed gradient,
-    which is then un-rotated in place: no slicing copies, no concatenation."""
+    which is then un-rotated in place: no slicing copies, no concatenation.  With grouped kv heads, or a sequence that is
+    not whole blocks of 128 tokens, the rotated blocks go into a tensor of their own and ``qkv`` stays as it is."""
 
     @staticmethod
     def forward(ctx, qkv, cos, sin, batch, seq, heads, kv_heads, d, causal, scale):
         from . import flash_attn_kernel as FK
         hd, kd = heads * d, kv_heads * d
-        K.rope_(qkv[:, :hd + kd], cos, sin, heads + kv_heads, d, seq)
-        q = qkv[:, :hd].view(batch, seq, heads, d)
-        k = qkv[:, hd:hd + kd].view(batch, seq, kv_heads, d)
+        qk = qkv
+        if heads == kv_heads and seq % 128 == 0:
+            K.rope_(qkv[:, :hd + kd], cos, sin, heads + kv_heads, d, seq)
+        else:
+            qk = K.rope(qkv[:, :hd + kd], cos, sin, heads + kv_heads, d, seq)
+        q = qk[:, :hd].view(batch, seq, heads, d)
+        k = qk[:, hd:hd + kd].view(batch, seq, kv_heads, d)
         v = qkv[:, hd + kd:].view(batch, seq, kv_heads, d)
         o, lse, _, _, _ = FK.fwd(q, k, v, causal, scale)
-        ctx.save_for_backward(qkv, o, lse, cos, sin)
+        ctx.save_for_backward(qk, qkv, o, lse, cos, sin)
         ctx.meta = (batch, seq, heads, kv_heads, d, causal, scale)
         return o
 
     @staticmethod
     def backward(ctx, do):
         from . import flash_attn_kernel as FK
-        qkv, o, lse, cos, sin = ctx.saved_tensors
+        qk, qkv, o, lse, cos, sin = ctx.saved_tensors
         batch, seq, heads, kv_heads, d, causal, scale = ctx.meta
         hd, kd = heads * d, kv_heads * d
-        q = qkv[:, :hd].view(batch, seq, heads, d)
-        k = qkv[:, hd:hd + kd].view(batch, seq, kv_heads, d)
+        q = qk[:, :hd].view(batch, seq, heads, d)
+        k = qk[:, hd:hd + kd].view(batch, seq, kv_heads, d)
         v = qkv[:, hd + kd:].view(batch, seq, kv_heads, d)
         dqkv = torch.empty_like(qkv)
         FK.bwd_into(do, q, k, v, o, lse, causal, scale, dqkv[:, :hd], dqkv[:, hd:hd + kd], dqkv[:, hd + kd:],
@@ -409,12 +410,11 @@ class _QkvRopeAttnFn(torch.autograd.Function):
 def qkv_rope_attention(qkv, cos, sin, batch, seq, heads, kv_heads, head_dim, causal=True, scale=None):
     """Attention output [batch, seq, heads, head_dim] from the packed projection ``qkv`` [batch*seq, (H+2Hk)*D]
     (q heads, then k heads, then v heads).  ``qkv`` is consumed: the kernel path rotates it in place."""
-    import math
     from . import flash_attn_kernel as FK
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     hd, kd = heads * head_dim, kv_heads * head_dim
     if (_use_kernel(qkv, fp16_ok=True) and qkv.is_contiguous() and head_dim == 128
-            and seq % 128 == 0 and heads == kv_heads and FK.available() and FK.has_strided_bwd()):
+            and heads % kv_heads == 0 and scale > 0 and FK.available() and FK.has_strided_bwd()):
         return _QkvRopeAttnFn.apply(qkv, cos, sin, batch, seq, heads, kv_heads, head_dim, bool(causal), float(scale))
     qk = rope(qkv[:, :hd + kd].contiguous(), cos, sin, heads + kv_heads, head_dim, seq)
     q = qk[:, :hd].reshape(batch, seq, heads, head_dim)

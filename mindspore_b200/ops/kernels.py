@@ -217,6 +217,21 @@ def rope_(x, cos, sin, heads, head_dim, seq, positions=None, backward=False):
     return x
 
 
+def rope(x, cos, sin, heads, head_dim, seq, backward=False, out=None):
+    """RoPE of x viewed as [tokens, heads * head_dim] (row pitch x.stride(-2)) into ``out`` (contiguous; a new
+    tensor by default)."""
+    x2 = x.reshape(-1, x.shape[-1]) if x.is_contiguous() else x
+    assert x2.dim() == 2 and x2.stride(1) == 1
+    tokens = x2.shape[0]
+    if out is None:
+        out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    rc = _fn("msb_rope_to", x2)(_p(x2), _p(out), _p(cos), _p(sin), None, tokens, heads, head_dim, x2.stride(0),
+                                out.shape[-1], seq, int(backward), _stream())
+    _native.check(rc, "rope")
+    _count()
+    return out
+
+
 def swiglu_fwd(gu):
     F = gu.shape[-1] // 2
     rows = gu.numel() // (2 * F)

@@ -65,6 +65,33 @@ def test_flash_attention_grouped_heads_and_odd_tiles(K, B, S, H, Hk, causal, dty
     _status_ok()
 
 
+@pytest.mark.parametrize("S,H,Hk", [(256, 4, 2), (200, 4, 4), (77, 4, 1)])
+def test_rotary_attention_keeps_its_input(K, S, H, Hk):
+    """RotaryFlashAttention with grouped heads or a ragged sequence: gradient against fp64, the packed projection left as it
+    was."""
+    from mindspore_b200.ops.llm_ops import RotaryFlashAttention
+    from mindspore_b200.ops import fused
+    D = 128
+    qkv = torch.randn(2 * S, (H + 2 * Hk) * D, device=DEV).bfloat16()
+    cos, sin = fused.rope_tables(S, D, device=DEV)
+    do = torch.randn(2 * S, H * D, device=DEV).bfloat16()
+    x = qkv.clone().requires_grad_(True)
+    y = RotaryFlashAttention(H, Hk, D)(x, cos, sin)
+    (g,) = torch.autograd.grad(y, x, do)
+    assert torch.equal(x.detach(), qkv)
+    r = qkv.double().requires_grad_(True)
+    q, k, v = (t.reshape(2, S, -1, D) for t in r.split([H * D, Hk * D, Hk * D], -1))
+    c, s = cos.double()[None, :, None], sin.double()[None, :, None]
+    rot = lambda t: torch.cat([t[..., :64] * c - t[..., 64:] * s, t[..., 64:] * c + t[..., :64] * s], -1)  # noqa: E731
+    p = torch.einsum("bqhd,bkhd->bhqk", rot(q), rot(k).repeat_interleave(H // Hk, 2)) / math.sqrt(D)
+    p = p.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), -math.inf)
+    ref = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(p, -1), v.repeat_interleave(H // Hk, 2)).reshape(2 * S, H * D)
+    ref.backward(do.double())
+    _near(y, ref, 6, torch.bfloat16)
+    _near(g, r.grad, 10, torch.bfloat16)
+    _status_ok()
+
+
 # ------------------------------------------------------------------------------------------------ cross entropy
 @pytest.mark.parametrize("rows,V", [(1, 1), (3, 7), (5, 4099), (64, 32000), (9, 50257)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
@@ -127,3 +154,37 @@ def test_norms_over_the_range_of_widths(K, rows, H, dtype):
     ref.backward(dy.double())
     for got, exp in ((y, ref), (dx, xd.grad), (dw, wd.grad), (db, bd.grad)):
         _near(got, exp, 2, dtype)
+
+
+# ------------------------------------------------------------------------------------------------ streaming kernels
+@pytest.mark.parametrize("rows,F", [(1, 8), (3, 24), (77, 11008), (1000, 1408)])
+def test_swiglu_sizes(K, rows, F):
+    gu, d = torch.randn(rows, 2 * F, device=DEV).bfloat16(), torch.randn(rows, F, device=DEV).bfloat16()
+    x = gu.double().requires_grad_(True)
+    ref = torch.nn.functional.silu(x[:, :F]) * x[:, F:]
+    ref.backward(d.double())
+    _near(K.swiglu_fwd(gu), ref, 2, torch.bfloat16)
+    _near(K.swiglu_bwd(gu, d), x.grad, 2, torch.bfloat16)
+
+
+@pytest.mark.parametrize("tokens,heads,D,seq", [(5, 1, 16, 5), (6, 3, 80, 3), (64, 9, 128, 32), (8, 40, 128, 8)])
+def test_rope_in_and_out_of_place(K, tokens, heads, D, seq):
+    """Widths that do not divide the block, odd numbers of heads, a pitch wider than the row, misaligned tables."""
+    wide = torch.randn(tokens, heads * D + 64, device=DEV).bfloat16()
+    x = wide[:, :heads * D]
+    ang = torch.randn(seq, D // 2, device=DEV)
+    store = torch.empty(2 * ang.numel() + 1, device=DEV)
+    cos, sin = (store[1 + i * ang.numel():1 + (i + 1) * ang.numel()].view_as(ang) for i in range(2))
+    cos.copy_(ang.cos())
+    sin.copy_(ang.sin())
+    p = torch.arange(tokens, device=DEV) % seq
+    c, s = cos.double()[p][:, None], sin.double()[p][:, None]
+    xd = x.double().view(tokens, heads, D)
+    a, b = xd[..., :D // 2], xd[..., D // 2:]
+    ref = torch.cat([a * c - b * s, b * c + a * s], -1).reshape(tokens, heads * D)
+    before = wide.clone()
+    _near(K.rope(x, cos, sin, heads, D, seq), ref, 2, torch.bfloat16)
+    assert torch.equal(wide, before)
+    K.rope_(x, cos, sin, heads, D, seq)
+    _near(x, ref, 2, torch.bfloat16)
+    assert torch.equal(wide[:, heads * D:], before[:, heads * D:])
