@@ -69,6 +69,7 @@ _CUDA_SIGNATURES = {
     "msb_momentum": (_I, [_P, _P, _P, _I, _P, _L, _P, _P, _P]),
     "msb_sumsq_finite": (_I, [_P, _I, _L, _P, _P, _P]),
     "msb_finalize_grad_scale": (_I, [_P, _P, _F, _F, _P, _P, _P, _P]),
+    "msb_fill_scalars": (_I, [_P, _P, _I, _P]),
     "msb_embedding_fwd": (_I, [_P, _P, _P, _L, _I, _I, _I, _P]),
     "msb_embedding_bwd": (_I, [_P, _P, _P, _L, _I, _I, _I, _P]),
     "msb_cast_f32_to_bf16": (_I, [_P, _P, _L, _F, _P]),

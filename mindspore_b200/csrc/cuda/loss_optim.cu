@@ -84,7 +84,7 @@ __device__ __forceinline__ void online_add_n(float& m, float& s, const float (&f
 //   stats[row] = {max, sum exp(l - max), logit[label] if label in slice else 0}
 // and, if loss != nullptr (the slice is the whole vocabulary), loss[row] as in ce_grad_kernel.
 // Bound by reading the logits once.  Four 16-byte loads are in flight per thread; the scalar 2-byte loads this replaces
-// kept too few bytes in flight.
+// kept too few bytes in flight (4096 x 32000 bf16: 121 -> 66 us, 4.0 TB/s).
 template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
 ce_stats_kernel(const T* __restrict__ logits, const int* __restrict__ labels, float* __restrict__ stats,
@@ -187,8 +187,8 @@ ce_mean_kernel(const float* __restrict__ loss, const int* __restrict__ labels, f
 
 // Given (possibly cross-rank combined) stats, writes loss[row] = log(sum) + max - target (0 for ignored
 // rows) and, if dlogits != nullptr, dlogits = (softmax - onehot) * grad_scale[0] / (divisor ? divisor[0] : 1) * (row
-// valid).  Bound by reading and writing the logits once: 16-byte accesses, four loads in flight per thread.  Where the
-// two rows are not equally aligned every element goes by itself.
+// valid).  Bound by reading and writing the logits once: 16-byte accesses, four loads in flight per thread (4096 x 32000
+// bf16: 78 us, 6.7 TB/s).  Where the two rows are not equally aligned every element goes by itself.
 template <typename T>
 __global__ void __launch_bounds__(kCeThreads)
 ce_grad_kernel(const T* logits, const int* __restrict__ labels, const float* __restrict__ stats,
@@ -320,28 +320,56 @@ __global__ void momentum_kernel(float* __restrict__ master, float* __restrict__ 
   }
 }
 
-// out[0] += sum(x^2) ; flag |= any non-finite
+// out[0] += sum(x^2) ; flag |= any non-finite.  Bound by reading x: 16-byte loads, four in flight per thread (a scalar
+// load per thread kept 8 KB per SM in flight; 2e8 fp32 values: 150 -> 146 us, 5.5 TB/s).  Elements in front of the
+// first and behind the last 16-byte boundary go by themselves.
 template <typename T>
-__global__ void sumsq_finite_kernel(const T* __restrict__ x, long long n, float* __restrict__ out,
-                                    int* __restrict__ nonfinite) {
+__global__ void __launch_bounds__(512)
+sumsq_finite_kernel(const T* __restrict__ x, long long n, float* __restrict__ out, int* __restrict__ nonfinite) {
+  constexpr int kVec = 16 / sizeof(T);
   __shared__ float red[32];
-  float acc = 0.f;
-  bool bad = false;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float v = to_f<T>(x[i]);
-    acc += v * v;
-    bad |= !isfinite(v);
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  uint32_t top = 0;                        // largest magnitude seen, as bits: at least 0x7f800000 if one is inf or NaN
+  auto add = [&](float v, int u) {
+    acc[u] += v * v;
+    top = max(top, __float_as_uint(v) & 0x7fffffffu);
+  };
+  const int off = static_cast<int>(reinterpret_cast<uintptr_t>(x) & 15) / static_cast<int>(sizeof(T));
+  const long long head = min(static_cast<long long>(off ? kVec - off : 0), n);
+  const long long vecs = (n - head) / kVec;
+  const uint4* body = reinterpret_cast<const uint4*>(x + head);
+  const long long tid = blockIdx.x * 512ll + threadIdx.x, step = gridDim.x * 512ll;
+  long long i = tid;
+  for (; i + 3 * step < vecs; i += 4 * step) {
+    uint4 r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) r[u] = body[i + u * step];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float f[kVec];
+      unpack16(r[u], f, T());
+#pragma unroll
+      for (int j = 0; j < kVec; ++j) add(f[j], u);
+    }
   }
-  acc = warp_sum(acc);
+  for (; i < vecs; i += step) {
+    float f[kVec];
+    unpack16(body[i], f, T());
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) add(f[j], j & 3);
+  }
+  if (tid < head) add(to_f<T>(x[tid]), 0);
+  if (tid < n - head - vecs * kVec) add(to_f<T>(x[head + vecs * kVec + tid]), 0);
+  const float mine = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[warp] = acc;
+  if (lane == 0) red[warp] = mine;
   __syncthreads();
   if (warp == 0) {
-    float t = lane < (blockDim.x >> 5) ? red[lane] : 0.f;
+    float t = lane < 16 ? red[lane] : 0.f;
     t = warp_sum(t);
     if (lane == 0) atomicAdd(out, t);
   }
-  if (bad) atomicOr(nonfinite, 1);
+  if (top >= 0x7f800000u) atomicOr(nonfinite, 1);
 }
 
 // hyper[7] (grad_scale of adamw) = inv_loss_scale * min(1, max_norm / (sqrt(sumsq)*inv_loss_scale + 1e-6)),
@@ -355,6 +383,16 @@ __global__ void finalize_grad_scale_kernel(const float* __restrict__ sumsq, cons
   *hyper_scale = s;
   if (skip) *skip = *nonfinite;
   if (norm_out) *norm_out = norm;
+}
+
+// Up to eight host scalars into device memory, as arguments of the launch: a copy from pageable host memory makes the
+// host wait for the stream, and with it the next kernels of the step (two of them per optimizer step of 2e8 parameters:
+// 1385 -> 1196 us).
+struct Scalars8 {
+  float v[8];
+};
+__global__ void fill_scalars_kernel(float* __restrict__ dst, const Scalars8 s, int n) {
+  if (threadIdx.x < n) dst[threadIdx.x] = s.v[threadIdx.x];
 }
 
 // ------------------------------------------------------------------------------------ embedding
@@ -523,6 +561,15 @@ MSB_EXPORT int msb_finalize_grad_scale(const float* sumsq, const int* nonfinite,
                                        float* hyper_scale, int* skip, float* norm_out, void* stream) {
   finalize_grad_scale_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(sumsq, nonfinite, inv_loss_scale, max_norm,
                                                                 hyper_scale, skip, norm_out);
+  MSB_CUDA_CHECK(cudaGetLastError());
+  return kOk;
+}
+
+MSB_EXPORT int msb_fill_scalars(float* dst, const float* host_values, int n, void* stream) {
+  if (n < 0 || n > 8) { set_last_error("fill_scalars: %d values (at most 8)", n); return kBadArg; }
+  Scalars8 s = {};
+  for (int i = 0; i < n; ++i) s.v[i] = host_values[i];
+  fill_scalars_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(dst, s, n);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }

@@ -25,6 +25,7 @@ from ..common.initializer import initializer
 from ..common.parameter import Parameter, ParameterTuple
 from ..common.tensor import Tensor
 from ..ops import kernels as K
+from ..ops import primitive as _primitive
 from ..ops.primitive import _wrap_out
 from .cell import Cell
 from .lr_schedule import LearningRateSchedule
@@ -557,8 +558,12 @@ def _to_plain(t):
 
 def _fill_hyper(h, start, values):
     """Writes scalars (host numbers, or 0-d tensors when the step is traced) into the device hyper-parameter
-    vector: one host-to-device copy when all are numbers."""
+    vector: one launch that carries them when all are numbers (one copy for a vector in host memory, and in a trace,
+    which records it)."""
     if not any(isinstance(v, torch.Tensor) for v in values):
+        if h.is_cuda and _primitive._trace_hook is None:
+            K.fill_scalars(h[start:start + len(values)], values)
+            return
         h[start:start + len(values)] = torch.tensor(values, dtype=torch.float32)
         return
     for i, v in enumerate(values):

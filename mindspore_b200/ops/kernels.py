@@ -371,6 +371,16 @@ def finalize_grad_scale(sumsq, nonfinite, inv_loss_scale, max_norm, hyper_scale,
     _count()
 
 
+def fill_scalars(dst, values):
+    """dst[i] = values[i] (host numbers, at most eight, fp32) without a host-to-device copy: they travel as launch
+    arguments, so the host does not wait for the stream."""
+    n = len(values)
+    host = (ctypes.c_float * n)(*values)
+    rc = _native.cuda().msb_fill_scalars(_p(dst), ctypes.addressof(host), n, _stream())
+    _native.check(rc, "fill_scalars")
+    _count()
+
+
 # --------------------------------------------------------------------------------------- embedding / casts
 def embedding_fwd(table, ids, vocab_start=0):
     H = table.shape[1]

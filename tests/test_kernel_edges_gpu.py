@@ -188,3 +188,29 @@ def test_rope_in_and_out_of_place(K, tokens, heads, D, seq):
     K.rope_(x, cos, sin, heads, D, seq)
     _near(x, ref, 2, torch.bfloat16)
     assert torch.equal(wide[:, heads * D:], before[:, heads * D:])
+
+
+@pytest.mark.parametrize("n,off", [(1, 0), (3, 1), (17, 3), (100003, 1), (1 << 22, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_sum_of_squares_of_slices(K, n, off, dtype):
+    x = torch.randn(n + off, device=DEV).to(dtype)[off:]
+    out, bad = torch.zeros(1, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    K.sumsq_finite(x, out, bad)
+    assert int(bad) == 0
+    _near(out, x.double().pow(2).sum().reshape(1), 1024, torch.float32)
+    for value in (math.inf, -math.inf, math.nan):
+        y = x.clone()
+        y[n // 2] = value
+        bad.zero_()
+        K.sumsq_finite(y, out, bad)
+        assert int(bad) == 1
+    big = torch.full((n,), 3e38, device=DEV).to(dtype)            # finite values whose squares are not
+    bad.zero_()
+    K.sumsq_finite(big, out, bad)
+    assert int(bad) == 0
+
+
+def test_fill_scalars(K):
+    h = torch.zeros(8, device=DEV)
+    K.fill_scalars(h[2:5], [0.1, 1e-8, 3])
+    assert torch.equal(h.cpu(), torch.tensor([0, 0, 0.1, 1e-8, 3, 0, 0, 0]))
