@@ -97,8 +97,12 @@ column_reduce_kernel(const elem_t* __restrict__ a, const elem_t* __restrict__ x,
 
 // stats: [2C] sums.  Writes scale/shift (and mean/rstd for backward); updates the moving statistics
 // moving = momentum * moving + (1 - momentum) * batch  (variance unbiased), as nn.BatchNorm2d does.
-__global__ void bn_finalize_kernel(const float* __restrict__ stats, const float* __restrict__ gamma,
-                                   const float* __restrict__ beta, float* __restrict__ moving_mean,
+// gamma / beta are fp32, or of the element type where `affine16`: no cast launches in front of these kernels.
+__device__ __forceinline__ float affine(const void* p, int c, int affine16) {
+  return affine16 ? e_to_f(static_cast<const elem_t*>(p)[c]) : static_cast<const float*>(p)[c];
+}
+__global__ void bn_finalize_kernel(const float* __restrict__ stats, const void* __restrict__ gamma,
+                                   const void* __restrict__ beta, int affine16, float* __restrict__ moving_mean,
                                    float* __restrict__ moving_var, float* __restrict__ scale,
                                    float* __restrict__ shift, float* __restrict__ mean_out,
                                    float* __restrict__ rstd_out, int C, float count, float momentum, float eps,
@@ -118,52 +122,77 @@ __global__ void bn_finalize_kernel(const float* __restrict__ stats, const float*
     var = moving_var[c];
   }
   const float r = rsqrtf(var + eps);
-  const float sc = gamma[c] * r;
+  const float sc = affine(gamma, c, affine16) * r;
   scale[c] = sc;
-  shift[c] = beta[c] - mean * sc;
+  shift[c] = affine(beta, c, affine16) - mean * sc;
   if (mean_out) {
     mean_out[c] = mean;
     rstd_out[c] = r;
   }
 }
 
+__device__ __forceinline__ void load_channels(const float* p, int c0, float (&f)[8]) {
+  *reinterpret_cast<float4*>(f) = *reinterpret_cast<const float4*>(p + c0);
+  *reinterpret_cast<float4*>(f + 4) = *reinterpret_cast<const float4*>(p + c0 + 4);
+}
+
+// Bound by its tensors' bytes.  Where the stride of the loop is a multiple of the row (every power-of-two channel count)
+// a thread stays on its eight channels: their coefficients are loaded once and no index is divided, and two positions are
+// in flight.
 __global__ void __launch_bounds__(kEwThreads)
 bn_apply_kernel(const elem_t* __restrict__ x, const float* __restrict__ scale, const float* __restrict__ shift,
                 const elem_t* __restrict__ residual, elem_t* __restrict__ y, long long total_vecs,
                 int vecs, int relu) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total_vecs;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c0 = (int)(i % vecs) * 8;
-    float v[8];
-    unpack8(reinterpret_cast<const uint4*>(x)[i], v);
-    const float4 sa = *reinterpret_cast<const float4*>(scale + c0), sb = *reinterpret_cast<const float4*>(scale + c0 + 4);
-    const float4 ha = *reinterpret_cast<const float4*>(shift + c0), hb = *reinterpret_cast<const float4*>(shift + c0 + 4);
-    const float sc[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
-    const float sh[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+  const long long step = (long long)gridDim.x * kEwThreads, first = blockIdx.x * (long long)kEwThreads + threadIdx.x;
+  const bool fixed = step % vecs == 0;
+  float sc[8], sh[8];
+  load_channels(scale, (int)(first % vecs) * 8, sc);
+  load_channels(shift, (int)(first % vecs) * 8, sh);
+  for (long long i = first; i < total_vecs; i += 2 * step) {
+    uint4 rx[2], rr[2];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = v[j] * sc[j] + sh[j];
-    if (residual) {
-      float rv[8];
-      unpack8(reinterpret_cast<const uint4*>(residual)[i], rv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] += rv[j];
+    for (int u = 0; u < 2; ++u) {
+      if (i + u * step < total_vecs) {
+        rx[u] = reinterpret_cast<const uint4*>(x)[i + u * step];
+        if (residual) rr[u] = reinterpret_cast<const uint4*>(residual)[i + u * step];
+      }
     }
-    if (relu) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.f);
+    for (int u = 0; u < 2; ++u) {
+      const long long k = i + u * step;
+      if (k < total_vecs) {
+        if (!fixed) {
+          load_channels(scale, (int)(k % vecs) * 8, sc);
+          load_channels(shift, (int)(k % vecs) * 8, sh);
+        }
+        float v[8];
+        unpack8(rx[u], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = v[j] * sc[j] + sh[j];
+        if (residual) {
+          float rv[8];
+          unpack8(rr[u], rv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] += rv[j];
+        }
+        if (relu) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.f);
+        }
+        reinterpret_cast<uint4*>(y)[k] = pack8(v);
+      }
     }
-    reinterpret_cast<uint4*>(y)[i] = pack8(v);
   }
 }
 
 // dx = gamma * rstd * (dy' - sum(dy')/count - xhat * sum(dy' xhat)/count) = A[c] * dy' + B[c] * x + D[c];
 // dres = dy' (optional).  coef = [A | B | D], each C floats.
-__global__ void bn_bwd_coeff_kernel(const float* __restrict__ gamma, const float* __restrict__ mean,
+__global__ void bn_bwd_coeff_kernel(const void* __restrict__ gamma, int affine16, const float* __restrict__ mean,
                                     const float* __restrict__ rstd, const float* __restrict__ sums,
                                     float* __restrict__ coef, int C, float inv_count) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  const float g = gamma[c], r = rstd[c], mu = mean[c];
+  const float g = affine(gamma, c, affine16), r = rstd[c], mu = mean[c];
   const float s1 = sums[c] * inv_count, s2 = sums[C + c] * inv_count;
   coef[c] = g * r;
   coef[C + c] = -g * r * r * s2;
@@ -175,30 +204,47 @@ bn_bwd_apply_kernel(const elem_t* __restrict__ dy, const elem_t* __restrict__ x,
                     const elem_t* __restrict__ y, const float* __restrict__ coef,
                     elem_t* __restrict__ dx, elem_t* __restrict__ dres, long long total_vecs, int vecs,
                     int C, int relu) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total_vecs;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c0 = (int)(i % vecs) * 8;
-    float g[8], xv[8];
-    unpack8(reinterpret_cast<const uint4*>(dy)[i], g);
-    unpack8(reinterpret_cast<const uint4*>(x)[i], xv);
-    if (relu) {
-      float yv[8];
-      unpack8(reinterpret_cast<const uint4*>(y)[i], yv);
+  const long long step = (long long)gridDim.x * kEwThreads, first = blockIdx.x * (long long)kEwThreads + threadIdx.x;
+  const bool fixed = step % vecs == 0;      // as in bn_apply_kernel
+  float ca[8], cb[8], cd[8];
+  auto coefficients = [&](long long k) {
+    const int c0 = (int)(k % vecs) * 8;
+    load_channels(coef, c0, ca);
+    load_channels(coef + C, c0, cb);
+    load_channels(coef + 2 * C, c0, cd);
+  };
+  coefficients(first);
+  for (long long i = first; i < total_vecs; i += 2 * step) {
+    uint4 rg[2], rx[2], ry[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] = yv[j] > 0.f ? g[j] : 0.f;
+    for (int u = 0; u < 2; ++u) {
+      const long long k = i + u * step;
+      if (k < total_vecs) {
+        rg[u] = reinterpret_cast<const uint4*>(dy)[k];
+        rx[u] = reinterpret_cast<const uint4*>(x)[k];
+        if (relu) ry[u] = reinterpret_cast<const uint4*>(y)[k];
+      }
     }
-    if (dres) reinterpret_cast<uint4*>(dres)[i] = pack8(g);
-    float ca[8], cb[8], cd[8];
-    *reinterpret_cast<float4*>(ca) = *reinterpret_cast<const float4*>(coef + c0);
-    *reinterpret_cast<float4*>(ca + 4) = *reinterpret_cast<const float4*>(coef + c0 + 4);
-    *reinterpret_cast<float4*>(cb) = *reinterpret_cast<const float4*>(coef + C + c0);
-    *reinterpret_cast<float4*>(cb + 4) = *reinterpret_cast<const float4*>(coef + C + c0 + 4);
-    *reinterpret_cast<float4*>(cd) = *reinterpret_cast<const float4*>(coef + 2 * C + c0);
-    *reinterpret_cast<float4*>(cd + 4) = *reinterpret_cast<const float4*>(coef + 2 * C + c0 + 4);
-    float o[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = ca[j] * g[j] + cb[j] * xv[j] + cd[j];
-    reinterpret_cast<uint4*>(dx)[i] = pack8(o);
+    for (int u = 0; u < 2; ++u) {
+      const long long k = i + u * step;
+      if (k < total_vecs) {
+        if (!fixed) coefficients(k);
+        float g[8], xv[8], o[8];
+        unpack8(rg[u], g);
+        unpack8(rx[u], xv);
+        if (relu) {
+          float yv[8];
+          unpack8(ry[u], yv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) g[j] = yv[j] > 0.f ? g[j] : 0.f;
+        }
+        if (dres) reinterpret_cast<uint4*>(dres)[k] = pack8(g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = ca[j] * g[j] + cb[j] * xv[j] + cd[j];
+        reinterpret_cast<uint4*>(dx)[k] = pack8(o);
+      }
+    }
   }
 }
 
@@ -347,12 +393,12 @@ MSB_EXPORT int MSB_FN(msb_channel_stats)(const void* x, float* out, long long ro
   return kOk;
 }
 
-MSB_EXPORT int MSB_FN(msb_bn_finalize)(const float* stats, const float* gamma, const float* beta, float* moving_mean,
-                               float* moving_var, float* scale, float* shift, float* mean_out, float* rstd_out, int C,
+MSB_EXPORT int MSB_FN(msb_bn_finalize)(const float* stats, const void* gamma, const void* beta, int affine16,
+                               float* moving_mean, float* moving_var, float* scale, float* shift, float* mean_out, float* rstd_out, int C,
                                float count, float momentum, float eps, int training, void* stream) {
   if (int rc = check_c("bn_finalize", C)) return rc;
-  bn_finalize_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(stats, gamma, beta, moving_mean, moving_var,
-                                                                         scale, shift, mean_out, rstd_out, C, count,
+  bn_finalize_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(stats, gamma, beta, affine16, moving_mean,
+                                                                         moving_var, scale, shift, mean_out, rstd_out, C, count,
                                                                          momentum, eps, training);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -363,7 +409,7 @@ MSB_EXPORT int MSB_FN(msb_bn_apply)(const void* x, const float* scale, const flo
   if (int rc = check_c("bn_apply", C)) return rc;
   if (rows <= 0) return kOk;
   const long long tv = rows * (C / 8);
-  bn_apply_kernel<<<ew_grid(tv), kEwThreads, 0, (cudaStream_t)stream>>>(
+  bn_apply_kernel<<<ew_grid((tv + 1) / 2), kEwThreads, 0, (cudaStream_t)stream>>>(
       (const elem_t*)x, scale, shift, (const elem_t*)residual, (elem_t*)y, tv, C / 8, relu);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
@@ -385,15 +431,15 @@ MSB_EXPORT int MSB_FN(msb_bn_bwd_reduce)(const void* dy, const void* x, const vo
 }
 
 // coef: fp32 [3C] scratch owned by the caller (filled here).
-MSB_EXPORT int MSB_FN(msb_bn_bwd_apply)(const void* dy, const void* x, const void* y, const float* gamma, const float* mean,
+MSB_EXPORT int MSB_FN(msb_bn_bwd_apply)(const void* dy, const void* x, const void* y, const void* gamma, int affine16, const float* mean,
                                 const float* rstd, const float* sums, float* coef, void* dx, void* dres,
                                 long long rows, int C, int relu, void* stream) {
   if (int rc = check_c("bn_bwd_apply", C)) return rc;
   if (rows <= 0) return kOk;
-  bn_bwd_coeff_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(gamma, mean, rstd, sums, coef, C,
+  bn_bwd_coeff_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(gamma, affine16, mean, rstd, sums, coef, C,
                                                                          1.f / (float)rows);
   const long long tv = rows * (C / 8);
-  bn_bwd_apply_kernel<<<ew_grid(tv), kEwThreads, 0, (cudaStream_t)stream>>>(
+  bn_bwd_apply_kernel<<<ew_grid((tv + 1) / 2), kEwThreads, 0, (cudaStream_t)stream>>>(
       (const elem_t*)dy, (const elem_t*)x, (const elem_t*)y, coef, (elem_t*)dx,
       (elem_t*)dres, tv, C / 8, C, relu);
   MSB_CUDA_CHECK(cudaGetLastError());

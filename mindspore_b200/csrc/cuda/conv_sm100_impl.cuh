@@ -26,7 +26,7 @@ namespace MSB_ELEM_NS {
 
 constexpr int kConvBM = 128;
 constexpr int kConvBK = 64;
-constexpr int kConvThreads = 192;
+constexpr int kConvThreads = 320;      // TMA warp, MMA warp, two epilogue groups of four warps
 constexpr int kMaxTaps = 49;
 constexpr int kMaxStatChannels = 2048;
 
@@ -42,6 +42,9 @@ struct ConvParams {
   int Cout, Cin;
   long long ldc;         // fwd: elements between output pixels; wgrad: elements between rows of dW
   int out_fp32, accumulate, ksplit;
+  // 1: output tiles go through swizzled shared memory and leave as TMA stores (wgrad: TMA reduce-adds); 0: per-thread
+  // stores / atomics, for fp32 forward outputs, channel counts and pitches that the tensor map cannot describe
+  int tma_out;
   short tap_map[kMaxTaps], tap_dh[kMaxTaps], tap_dw[kMaxTaps];
 };
 
@@ -56,37 +59,38 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* t
 
 template <int BN>
 struct ConvCfg {
-  static constexpr int kStages = (BN == 256) ? 4 : 6;
+  static constexpr int kStages = (BN == 256) ? 3 : 5;
   static constexpr int kABytes = kConvBM * kConvBK * 2;
   static constexpr int kBBytes = BN * kConvBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kBarOffset = kStages * kStageBytes;
+  // epilogue staging: 8 warps x (32 rows x 128 B), 1024-byte aligned behind the stage ring
+  static constexpr int kStagingOffset = kStages * kStageBytes;
+  static constexpr int kBarOffset = kStagingOffset + 8 * 4096;
   static constexpr int kStatOffset = kBarOffset + 256;
   static constexpr int kSmemBytes = kStatOffset + 2 * kMaxStatChannels * 4 + 1024;
 };
 
-// Sum over the 32 lanes of a warp of v[j], for every j: afterwards lane j holds the total of column j in v[0].
-__device__ __forceinline__ float warp_column_sums(float (&v)[32], int lane) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const bool upper = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < off; ++i) {
-      const float send = upper ? v[i] : v[i + off];
-      const float keep = upper ? v[i + off] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  return v[0];
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* tmap, const void* smem_src, int c, int w, int h, int n) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap)),
+               "r"(smem_u32(smem_src)), "r"(c), "r"(w), "r"(h), "r"(n)
+               : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tmap, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
 }
 
 template <int BN, bool WGRAD>
 __global__ void __launch_bounds__(kConvThreads, 1)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant__ CUtensorMap tmX1,
                   const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
-                  const __grid_constant__ CUtensorMap tmO, const ConvParams p) {
+                  const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmY, const ConvParams p) {
   // tmX*: input activations (parity planes).  tmO: fwd = weights [Cout, taps*Cin] (3-D map, K-major);
-  // wgrad = dY (4-D map).
+  // wgrad = dY (4-D map).  tmY: the output (fwd 4-D, boxes of 64 channels x 32 pixels; wgrad dW as a matrix, boxes of
+  // 32 x 32), valid when p.tma_out.
   using Cfg = ConvCfg<BN>;
   constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -103,7 +107,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
   volatile int* consumed_cnt = cta_abort + 2;
   float* s_stats = reinterpret_cast<float*>(smem + Cfg::kStatOffset);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const AbortCtx ab{cta_abort, p.status};
   const CUtensorMap* maps[4] = {&tmX0, &tmX1, &tmX2, &tmX3};
@@ -145,7 +149,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   // tile -> (outer index, m block, n block); m fastest so that CTAs running together share the weight tile
   auto tile_coords = [&](int tile, int& o, int& m_blk, int& n_blk) {
@@ -219,51 +223,86 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc = umma_idesc_elem(kConvBM, BN, WGRAD, WGRAD);
-      int s = 0;
-      uint32_t ph = 0;
-      int it = 0;
-      int consumed = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-        int o, m_blk, n_blk, kb_lo, kb_hi;
-        tile_coords(tile, o, m_blk, n_blk);
-        k_range(o, kb_lo, kb_hi);
-        const int acc = it & 1;
-        const uint32_t acc_ph = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1, ab)) { ok = false; break; }
+    // -------------------------------------------------------------------- MMA issuer (whole warp, one elected lane)
+    constexpr uint32_t idesc = umma_idesc_elem(kConvBM, BN, WGRAD, WGRAD);
+    const uint32_t lead = elect_one();
+    const uint64_t a_desc = umma_smem_desc(smem_u32(smem_a), WGRAD ? 8192 : 16, 1024);
+    const uint64_t b_desc = umma_smem_desc(smem_u32(smem_b), WGRAD ? 8192 : 16, 1024);
+    int s = 0;
+    uint32_t ph = 0;
+    int it = 0;
+    int consumed = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      int o, m_blk, n_blk, kb_lo, kb_hi;
+      tile_coords(tile, o, m_blk, n_blk);
+      k_range(o, kb_lo, kb_hi);
+      const int acc = it & 1;
+      const uint32_t acc_ph = (it >> 1) & 1;
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_ph ^ 1, ab)) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_warp(&full_bar[s], ph, ab)) { ok = false; break; }
+        ++consumed;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
-          if (!mbar_wait(&full_bar[s], ph, ab)) { ok = false; break; }
-          ++consumed;
+        const uint64_t ad = a_desc + s * (Cfg::kABytes >> 4), bd = b_desc + s * (Cfg::kBBytes >> 4);
+        if (lead) {
           *consumed_cnt = consumed;
-          tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem_a + s * Cfg::kABytes);
-          const uint32_t b_addr = smem_u32(smem_b + s * Cfg::kBBytes);
 #pragma unroll
-          for (int kk = 0; kk < kConvBK / 16; ++kk) {
-            const uint64_t adesc = WGRAD ? umma_smem_desc(a_addr + kk * 2048, 8192, 1024)
-                                         : umma_smem_desc(a_addr + kk * 32, 16, 1024);
-            const uint64_t bdesc = WGRAD ? umma_smem_desc(b_addr + kk * 2048, 8192, 1024)
-                                         : umma_smem_desc(b_addr + kk * 32, 16, 1024);
-            umma_bf16(d_tmem, adesc, bdesc, idesc, (kb != kb_lo) || (kk != 0));
-          }
+          for (int kk = 0; kk < kConvBK / 16; ++kk)
+            umma_bf16(d_tmem, ad + kk * (WGRAD ? 128 : 2), bd + kk * (WGRAD ? 128 : 2), idesc, (kb != kb_lo) || (kk != 0));
           umma_commit(&empty_bar[s]);
-          if (++s == kStages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(&tfull_bar[acc]);
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1; }
       }
+      if (ok && lead) umma_commit(&tfull_bar[acc]);
+      __syncwarp();
     }
     __syncwarp();
   } else {
-    // -------------------------------------------------------------------- epilogue (warps 2-5)
-    const int q = warp & 3;
-    int it = 0;
+    // -------------------------------------------------------------------- epilogue
+    // Two groups of four warps take the tiles in turn, each on its own accumulator.  A 1x1 convolution of 256 channels
+    // has about 2700 cycles per tile from HBM's side; one group with per-thread row stores needed four times that.
+    // 64 x 56 x 56 pixels, 64 -> 256 and back: 64 -> 31 us each; weight gradients, whose tiles left as fp32 atomics of
+    // single elements: 88 -> 29 us (1x1, 256 columns) and 91 -> 62 us (128 columns).
+    const int q = warp & 3, grp = (warp - 2) >> 2;
+    int it = grp;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+    uint8_t* staging = smem + Cfg::kStagingOffset + (warp - 2) * 4096;
+    const int sw = lane & 7;
+    uint8_t* rowp = staging + lane * 128;
+    bool pending = false;
+    auto staging_free = [&]() {           // the store that reads the staging buffer has read it
+      if (pending) {
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+      }
+      pending = true;
+    };
+    // statistics of this lane's two columns of every 64-column chunk, flushed when the column block changes
+    float st[BN / 64][4];
+#pragma unroll
+    for (int c = 0; c < BN / 64; ++c)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) st[c][j] = 0.f;
+    int st_n0 = -1;
+    auto flush_stats = [&]() {
+#pragma unroll
+      for (int c = 0; c < BN / 64; ++c) {
+        const int col = st_n0 + c * 64 + lane * 2;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (col + j < p.Cout) {
+            atomicAdd(&s_stats[col + j], st[c][j]);
+            atomicAdd(&s_stats[p.Cout + col + j], st[c][2 + j]);
+          }
+          st[c][j] = st[c][2 + j] = 0.f;
+        }
+      }
+    };
+    for (int tile = blockIdx.x + grp * gridDim.x; tile < total_tiles && ok; tile += 2 * gridDim.x, it += 2) {
       int o, m_blk, n_blk, kb_lo, kb_hi;
       tile_coords(tile, o, m_blk, n_blk);
       k_range(o, kb_lo, kb_hi);
@@ -276,6 +315,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       bool row_ok;
       long long c_off;
+      int bw0 = 0, bh0 = 0, bn0 = 0;       // origin of this warp's 32 pixels
       if (WGRAD) {
         const int co = m_blk * kConvBM + r;
         row_ok = co < p.Cout && kb_lo < kb_hi;
@@ -286,67 +326,118 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
         const int n = n0 + r / (p.tw * p.th), h = h0 + (r / p.tw) % p.th, w = w0 + r % p.tw;
         row_ok = n < p.N && h < p.Ho && w < p.Wo;
         c_off = ((static_cast<long long>(n) * p.Ho + h) * p.Wo + w) * p.ldc;
+        const int r0 = q * 32;
+        bn0 = n0 + r0 / (p.tw * p.th);
+        bh0 = h0 + (r0 / p.tw) % p.th;
+        bw0 = w0 + r0 % p.tw;
       }
-#pragma unroll 1
-      for (int c = 0; c < BN; c += 32) {
-        if (nc0 + c >= gemm_n) break;  // warp-uniform
-        uint32_t rr[32];
-        tmem_ld_32x32(t_row + c, rr);
-        tmem_ld_wait();
-        const int col0 = nc0 + c;
-        float v[32];
+      if (!WGRAD && p.tma_out) {
+        if (want_stats && st_n0 != nc0) {
+          if (st_n0 >= 0) flush_stats();
+          st_n0 = nc0;
+        }
+        const bool box_ok = bn0 < p.N && bh0 < p.Ho && bw0 < p.Wo;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = row_ok ? __uint_as_float(rr[j]) : 0.f;
-        if (WGRAD || p.out_fp32) {
-          float* dst = static_cast<float*>(p.C) + c_off + col0;
-          if (row_ok) {
-            if (WGRAD && (p.ksplit > 1 || p.accumulate)) {
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < gemm_n) atomicAdd(dst + j, v[j]);
-            } else {
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < gemm_n) dst[j] = v[j];
-            }
+        for (int c = 0; c < BN / 64; ++c) {
+          const int col0 = nc0 + c * 64;
+          if (col0 >= gemm_n) break;       // warp-uniform
+          uint32_t rr[2][32];
+          tmem_ld_32x32(t_row + c * 64, rr[0]);
+          tmem_ld_32x32(t_row + c * 64 + 32, rr[1]);
+          tmem_ld_wait();
+          staging_free();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t* e = &rr[j >> 2][(j & 3) * 8];
+            uint4 ov;
+            ov.x = pack_e2(__uint_as_float(e[0]), __uint_as_float(e[1]));
+            ov.y = pack_e2(__uint_as_float(e[2]), __uint_as_float(e[3]));
+            ov.z = pack_e2(__uint_as_float(e[4]), __uint_as_float(e[5]));
+            ov.w = pack_e2(__uint_as_float(e[6]), __uint_as_float(e[7]));
+            if (!row_ok) ov = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(rowp + ((j ^ sw) << 4)) = ov;
           }
-        } else {
-          elem_t* dst = static_cast<elem_t*>(p.C) + c_off + col0;
-          const bool full = (col0 + 32 <= gemm_n);
-          if (row_ok) {
-            if (full && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 ov;
-                ov.x = pack_e2(v[j], v[j + 1]);
-                ov.y = pack_e2(v[j + 2], v[j + 3]);
-                ov.z = pack_e2(v[j + 4], v[j + 5]);
-                ov.w = pack_e2(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = ov;
-              }
-            } else {
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < gemm_n) dst[j] = f_to_e(v[j]);
-            }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && box_ok) {
+            tma_store_4d(&tmY, staging, col0, bw0, bh0, bn0);
+            tma_store_commit();
           }
           if (want_stats) {
-            // statistics of what was stored (the rounded values); rows outside the image contribute zero
-            float sq[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              v[j] = e_to_f(f_to_e(v[j]));
-              sq[j] = v[j] * v[j];
+            // of what was stored (the rounded values); rows outside the image contribute zero.  Lane l sums columns 2l and
+            // 2l + 1 down the 32 staged rows: 32 conflict-free loads instead of 124 shuffles.
+#pragma unroll 8
+            for (int rw = 0; rw < 32; ++rw) {
+              const float2 v = e2_to_f2(*reinterpret_cast<const elem2_t*>(staging + rw * 128 + (((lane >> 2) ^ (rw & 7)) << 4) +
+                                                                         (lane & 3) * 4));
+              st[c][0] += v.x;
+              st[c][1] += v.y;
+              st[c][2] += v.x * v.x;
+              st[c][3] += v.y * v.y;
             }
-            const float s1 = warp_column_sums(v, lane);
-            const float s2 = warp_column_sums(sq, lane);
-            if (col0 + lane < p.Cout) {
-              atomicAdd(&s_stats[col0 + lane], s1);
-              atomicAdd(&s_stats[p.Cout + col0 + lane], s2);
+            __syncwarp();
+          }
+        }
+      } else if (WGRAD && p.tma_out) {
+        const int row0 = m_blk * kConvBM + q * 32, x0 = (o / p.ksplit) * p.Cin;
+        const bool box_ok = row0 < p.Cout && kb_lo < kb_hi;
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 32) {
+          if (nc0 + c >= gemm_n || !box_ok) break;     // warp-uniform
+          uint32_t rr[32];
+          tmem_ld_32x32(t_row + c, rr);
+          tmem_ld_wait();
+          staging_free();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(rowp + ((j ^ sw) << 4)) = make_uint4(rr[4 * j], rr[4 * j + 1], rr[4 * j + 2],
+                                                                           rr[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_3d(&tmY, staging, x0 + nc0 + c, row0, 0);
+            tma_store_commit();
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN; c += 32) {
+          if (nc0 + c >= gemm_n) break;  // warp-uniform
+          uint32_t rr[32];
+          tmem_ld_32x32(t_row + c, rr);
+          tmem_ld_wait();
+          const int col0 = nc0 + c;
+          if (row_ok && (WGRAD || p.out_fp32)) {
+            float* dst = static_cast<float*>(p.C) + c_off + col0;
+            if (WGRAD && (p.ksplit > 1 || p.accumulate)) {
+              for (int j = 0; j < 32; ++j)
+                if (col0 + j < gemm_n) atomicAdd(dst + j, __uint_as_float(rr[j]));
+            } else {
+              for (int j = 0; j < 32; ++j)
+                if (col0 + j < gemm_n) dst[j] = __uint_as_float(rr[j]);
+            }
+          } else if (row_ok) {
+            elem_t* dst = static_cast<elem_t*>(p.C) + c_off + col0;
+            for (int j = 0; j < 32; ++j) {
+              if (col0 + j < gemm_n) {
+                const elem_t e = f_to_e(__uint_as_float(rr[j]));
+                dst[j] = e;
+                if (want_stats) {
+                  const float v = e_to_f(e);
+                  atomicAdd(&s_stats[col0 + j], v);
+                  atomicAdd(&s_stats[p.Cout + col0 + j], v * v);
+                }
+              }
             }
           }
+          __syncwarp();
         }
       }
       tc_fence_before_sync();
       mbar_arrive(&tempty_bar[acc]);
     }
+    if (want_stats && st_n0 >= 0) flush_stats();
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
   // ---------------------------------------------------------------------- teardown
@@ -431,7 +522,7 @@ int setup_input(CUtensorMap maps[4], ConvParams* p, const void* x, int N, int H,
 }
 
 template <int BN, bool WGRAD>
-int launch_conv(const CUtensorMap maps[4], const CUtensorMap& tmO, const ConvParams& p, int tiles,
+int launch_conv(const CUtensorMap maps[4], const CUtensorMap& tmO, const CUtensorMap& tmY, const ConvParams& p, int tiles,
                 cudaStream_t stream) {
   using Cfg = ConvCfg<BN>;
   auto kern = conv_igemm_kernel<BN, WGRAD>;
@@ -441,7 +532,7 @@ int launch_conv(const CUtensorMap maps[4], const CUtensorMap& tmO, const ConvPar
     configured = true;
   }
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, kConvThreads, Cfg::kSmemBytes, stream>>>(maps[0], maps[1], maps[2], maps[3], tmO, p);
+  kern<<<grid, kConvThreads, Cfg::kSmemBytes, stream>>>(maps[0], maps[1], maps[2], maps[3], tmO, tmY, p);
   MSB_CUDA_CHECK(cudaGetLastError());
   return kOk;
 }
@@ -480,11 +571,21 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
   const int bn = (Cout <= 128 || pix_tiles * ((Cout + 255) / 256) < sm_count()) ? 128 : 256;
   const long long K = static_cast<long long>(R) * S * Cin;
   if (int rc = encode_tmap_3d(&tmW, w, 2, K, Cout, 1, K * 2, K * 2 * Cout, 64, bn, 1)) return rc;
+  // the output as TMA sees it: a warp's 32 rows are a sub-box of the tile's (all extents are powers of two)
+  CUtensorMap tmY = tmW;
+  if (!out_fp32 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && ldy % 8 == 0) {
+    const uint32_t bw = p.tw < 32 ? p.tw : 32, bh = p.th < 32 / (int)bw ? p.th : 32 / bw;
+    const uint32_t ybox[4] = {64u, bw, bh, 32u / (bw * bh)};
+    const uint64_t ydims[4] = {(uint64_t)Cout, (uint64_t)Wo, (uint64_t)Ho, (uint64_t)N};
+    const uint64_t yst[3] = {(uint64_t)(ldy * 2), (uint64_t)(Wo * ldy * 2), (uint64_t)((long long)Ho * Wo * ldy * 2)};
+    if (int rc = encode_tmap_4d(&tmY, y, ydims, yst, ybox)) return rc;
+    p.tma_out = 1;
+  }
   const long long tiles = pix_tiles * ((Cout + bn - 1) / bn);
   if (tiles > 0x7fffffffLL) { set_last_error("conv_fwd: too many tiles"); return kTooLarge; }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (bn == 256) return launch_conv<256, false>(maps, tmW, p, (int)tiles, stream);
-  return launch_conv<128, false>(maps, tmW, p, (int)tiles, stream);
+  if (bn == 256) return launch_conv<256, false>(maps, tmW, tmY, p, (int)tiles, stream);
+  return launch_conv<128, false>(maps, tmW, tmY, p, (int)tiles, stream);
 }
 
 // dw[Cout, R, S, Cin] (fp32) (+)= sum over pixels of dy[N, Ho, Wo, Cout] x shifted x[N, H, W, Cin].
@@ -513,16 +614,26 @@ MSB_EXPORT int MSB_FN(msb_conv_wgrad)(const void* x, const void* dy, float* dw, 
   const int bn = Cin <= 128 ? 128 : 256;
   const long long base_tiles = static_cast<long long>((Cout + kConvBM - 1) / kConvBM) * ((Cin + bn - 1) / bn) * p.taps;
   const long long pix_tiles = static_cast<long long>(p.tiles_w) * p.tiles_h * p.tiles_n;
-  long long split = (2LL * sm_count() + base_tiles - 1) / base_tiles;
-  if (split > pix_tiles) split = pix_tiles;
-  if (split < 1) split = 1;
+  // Split of the pixel loop with the fewest k-blocks on the longest CTA: rounds of one tile per SM, each as long as its
+  // k-blocks plus about eight for filling the pipeline and adding the tile into dW.
+  long long split = 1, best = -1;
+  for (long long t = 1; t <= pix_tiles && (t == 1 || base_tiles * (t - 1) < 2LL * sm_count()); ++t) {
+    const long long rounds = (base_tiles * t + sm_count() - 1) / sm_count(), cost = rounds * ((pix_tiles + t - 1) / t + 8);
+    if (best < 0 || cost < best) { best = cost; split = t; }
+  }
   p.ksplit = static_cast<int>(split);
+  CUtensorMap tmY = tmDY;
+  if (Cin % 32 == 0 && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) {
+    if (int rc = encode_tmap_3d(&tmY, dw, 4, (uint64_t)p.ldc, Cout, 1, p.ldc * 4, (uint64_t)p.ldc * 4 * Cout, 32, 32, 1))
+      return rc;
+    p.tma_out = 1;
+  }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (!accumulate)
     MSB_CUDA_CHECK(cudaMemsetAsync(dw, 0, sizeof(float) * static_cast<size_t>(Cout) * R * S * Cin, stream));
   const long long tiles = base_tiles * split;
-  if (bn == 256) return launch_conv<256, true>(maps, tmDY, p, (int)tiles, stream);
-  return launch_conv<128, true>(maps, tmDY, p, (int)tiles, stream);
+  if (bn == 256) return launch_conv<256, true>(maps, tmDY, tmY, p, (int)tiles, stream);
+  return launch_conv<128, true>(maps, tmDY, tmY, p, (int)tiles, stream);
 }
 
 namespace msb {

@@ -23,10 +23,10 @@ _native.register_cuda_signature("msb_conv_fwd", _I, [_P, _P, _P, _P] + [_I] * 13
 _native.register_cuda_signature("msb_conv_wgrad", _I, [_P, _P, _P] + [_I] * 12 + [_L, _L, _I, _P])
 _native.register_cuda_signature("msb_im2col_nhwc", _I, [_P, _P] + [_I] * 12 + [_P])
 _native.register_cuda_signature("msb_channel_stats", _I, [_P, _P, _L, _I, _P])
-_native.register_cuda_signature("msb_bn_finalize", _I, [_P] * 9 + [_I, _F, _F, _F, _I, _P])
+_native.register_cuda_signature("msb_bn_finalize", _I, [_P] * 3 + [_I] + [_P] * 6 + [_I, _F, _F, _F, _I, _P])
 _native.register_cuda_signature("msb_bn_apply", _I, [_P, _P, _P, _P, _P, _L, _I, _I, _P])
 _native.register_cuda_signature("msb_bn_bwd_reduce", _I, [_P, _P, _P, _P, _P, _P, _L, _I, _I, _P])
-_native.register_cuda_signature("msb_bn_bwd_apply", _I, [_P] * 10 + [_L, _I, _I, _P])
+_native.register_cuda_signature("msb_bn_bwd_apply", _I, [_P] * 4 + [_I] + [_P] * 6 + [_L, _I, _I, _P])
 _native.register_cuda_signature("msb_maxpool3x3s2", _I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P])
 _native.register_cuda_signature("msb_global_avgpool", _I, [_P, _P, _I, _I, _I, _I, _P])
 
@@ -214,6 +214,13 @@ def conv2d(x, w, stride, pads, dilation=(1, 1), bias=None):
 
 
 # ------------------------------------------------------------------------------------------------ BatchNorm (+ ReLU)
+def _affine(x, gamma, beta):
+    """gamma and beta as the BatchNorm kernels take them: both of x's 16-bit type (flag 1) or both fp32 (flag 0)."""
+    if gamma.dtype == beta.dtype == x.dtype and gamma.is_contiguous() and beta.is_contiguous():
+        return gamma, beta, 1
+    return gamma.float().contiguous(), beta.float().contiguous(), 0
+
+
 class _BnActFn(torch.autograd.Function):
     """y = relu(bn(x) (+ residual)) in training mode from precomputed channel sums of x.
 
@@ -224,42 +231,38 @@ class _BnActFn(torch.autograd.Function):
     def forward(ctx, x, stats, gamma, beta, residual, relu, eps, moving):
         n, c, h, w = x.shape
         rows = n * h * w
-        dev = x.device
-        scale = torch.empty(c, dtype=torch.float32, device=dev)
-        shift = torch.empty(c, dtype=torch.float32, device=dev)
-        mean = torch.empty(c, dtype=torch.float32, device=dev)
-        rstd = torch.empty(c, dtype=torch.float32, device=dev)
+        scale, shift, mean, rstd = torch.empty((4, c), dtype=torch.float32, device=x.device).unbind(0)
         mm, mv, momentum = moving
-        g32, b32 = gamma.float().contiguous(), beta.float().contiguous()
-        lib = _native.cuda()
-        _native.check(lib.msb_bn_finalize(_p(stats), _p(g32), _p(b32), _p(mm), _p(mv), _p(scale), _p(shift), _p(mean),
-                                          _p(rstd), c, float(rows), float(momentum), float(eps), 1, _stream()),
+        g, b, affine16 = _affine(x, gamma, beta)
+        _native.check(K._fn("msb_bn_finalize", x)(_p(stats), _p(g), _p(b), affine16, _p(mm), _p(mv), _p(scale), _p(shift),
+                                                  _p(mean), _p(rstd), c, float(rows), float(momentum), float(eps), 1,
+                                                  _stream()),
                       "bn_finalize")
         y = torch.empty_like(x, memory_format=CL)
         res = _nhwc(residual) if residual is not None else None
         _native.check(K._fn("msb_bn_apply", x)(_p(x), _p(scale), _p(shift), _p(res), _p(y), rows, c, int(relu), _stream()),
                       "bn_apply")
         _count(2)
-        ctx.save_for_backward(x, y, g32, mean, rstd)
-        ctx.relu, ctx.has_res = relu, residual is not None
+        ctx.save_for_backward(x, y, g, mean, rstd)
+        ctx.relu, ctx.has_res, ctx.affine16 = relu, residual is not None, affine16
         ctx.gamma_ref, ctx.beta_ref = gamma, beta
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, y, g32, mean, rstd = ctx.saved_tensors
+        x, y, g, mean, rstd = ctx.saved_tensors
         n, c, h, w = x.shape
         rows = n * h * w
         dy = _nhwc(dy)
         sums = torch.zeros(2 * c, dtype=torch.float32, device=x.device)
-        lib = _native.cuda()
         _native.check(K._fn("msb_bn_bwd_reduce", x)(_p(dy), _p(x), _p(y), _p(mean), _p(rstd), _p(sums), rows, c,
                                             int(ctx.relu), _stream()), "bn_bwd_reduce")
         dx = torch.empty_like(x, memory_format=CL)
         dres = torch.empty_like(x, memory_format=CL) if ctx.has_res else None
         coef = torch.empty(3 * c, dtype=torch.float32, device=x.device)
-        _native.check(K._fn("msb_bn_bwd_apply", x)(_p(dy), _p(x), _p(y), _p(g32), _p(mean), _p(rstd), _p(sums), _p(coef),
-                                           _p(dx), _p(dres), rows, c, int(ctx.relu), _stream()), "bn_bwd_apply")
+        _native.check(K._fn("msb_bn_bwd_apply", x)(_p(dy), _p(x), _p(y), _p(g), ctx.affine16, _p(mean), _p(rstd), _p(sums),
+                                                    _p(coef), _p(dx), _p(dres), rows, c, int(ctx.relu), _stream()),
+                      "bn_bwd_apply")
         _count(3)
         dgamma, dbeta = sums[c:], sums[:c]
         out_g = out_b = None
@@ -291,10 +294,10 @@ def bn_act_inference(x, gamma, beta, moving_mean, moving_var, relu=True, residua
     dev = x.device
     scale = torch.empty(c, dtype=torch.float32, device=dev)
     shift = torch.empty(c, dtype=torch.float32, device=dev)
-    lib = _native.cuda()
-    _native.check(lib.msb_bn_finalize(None, _p(gamma.float().contiguous()), _p(beta.float().contiguous()),
-                                      _p(moving_mean), _p(moving_var), _p(scale), _p(shift), None, None, c, 1.0, 0.0,
-                                      float(eps), 0, _stream()), "bn_finalize")
+    g, b, affine16 = _affine(x, gamma, beta)
+    _native.check(K._fn("msb_bn_finalize", x)(None, _p(g), _p(b), affine16, _p(moving_mean), _p(moving_var), _p(scale),
+                                              _p(shift), None, None, c, 1.0, 0.0, float(eps), 0, _stream()),
+                  "bn_finalize")
     y = torch.empty_like(x, memory_format=CL)
     res = _nhwc(residual) if residual is not None else None
     _native.check(K._fn("msb_bn_apply", x)(_p(x), _p(scale), _p(shift), _p(res), _p(y), n * h * w, c, int(relu), _stream()),

@@ -214,3 +214,25 @@ def test_fill_scalars(K):
     h = torch.zeros(8, device=DEV)
     K.fill_scalars(h[2:5], [0.1, 1e-8, 3])
     assert torch.equal(h.cpu(), torch.tensor([0, 0, 0.1, 1e-8, 3, 0, 0, 0]))
+
+
+# ------------------------------------------------------------------------------------------------ convolution
+@pytest.mark.parametrize("N,C,H,W,Cout,k,stride", [(1, 64, 7, 7, 64, 3, 1), (3, 64, 13, 9, 256, 1, 1),
+                                                  (2, 128, 15, 15, 128, 3, 2), (5, 64, 3, 5, 320, 1, 1)])
+def test_convolution_edges(K, N, C, H, W, Cout, k, stride):
+    """Pixel tiles that overhang the image on every side, one and several column blocks: output, the statistics that the
+    epilogue gathers, and the weight gradient."""
+    from mindspore_b200.ops import conv_kernel as CK
+    x = torch.randn(N, C, H, W, device=DEV).bfloat16().to(memory_format=torch.channels_last)
+    w = (torch.randn(Cout, C, k, k, device=DEV) / math.sqrt(C * k * k)).bfloat16()
+    y, stats = CK._ConvFn.apply(x, w, stride, k // 2, k // 2, True)
+    ref = torch.nn.functional.conv2d(x.double(), w.double(), None, stride, k // 2)
+    _near(y, ref, 2, torch.bfloat16)
+    yd = y.double()
+    _near(stats[:Cout], yd.sum((0, 2, 3)), 4096, torch.float32)
+    _near(stats[Cout:], yd.pow(2).sum((0, 2, 3)), 4096, torch.float32)
+    dy = torch.randn_like(ref).bfloat16().to(memory_format=torch.channels_last)
+    dw = CK.conv_wgrad_raw(x, dy, k, k, stride, k // 2, k // 2).permute(0, 3, 1, 2)
+    refw = torch.nn.grad.conv2d_weight(x.double(), w.shape, dy.double(), stride, k // 2)
+    _near(dw, refw, 1024, torch.float32)
+    _status_ok()
