@@ -1,4 +1,4 @@
-// bf16 GEMM on CTA pairs: tcgen05.mma.cta_group::2, one 256 x 256 output tile per two SMs.
+// 16-bit GEMM on CTA pairs: tcgen05.mma.cta_group::2, one 256 x 256 output tile per two SMs, batched.
 //
 //   C[m][n] (+)= sum_k A[m][k] * B[n][k]       (operand storage flags as in gemm_sm100.cu)
 //
@@ -41,9 +41,9 @@ constexpr int k2SmemBytes = k2BarOffset + 512 + 1024;
 struct Gemm2Params {
   const void* bias;
   int* status;
-  int* debug;          // optional: [4] tensor-memory addresses returned to rank 0 / rank 1
-  int M, N, K;
+  int M, N, K, batch;
   int out_fp32, accumulate;
+  int fp16;            // operands, bias and a 16-bit output are fp16 instead of bf16
   float alpha;
   // split-K: every output tile is ksplit work items, item j covering k-blocks [j, j+1) * num_kb / ksplit; each item
   // adds its partial product into C with the TMA reduce epilogue (fp32 accumulate only).  It shortens the last,
@@ -163,7 +163,7 @@ __device__ __forceinline__ void tma_reduce_add_3d_2(const CUtensorMap* tmap, con
                : "memory");
 }
 
-template <bool A_MN, bool B_MN, int ACC>
+template <bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(k2Threads, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const Gemm2Params p) {
@@ -178,9 +178,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank();
+  const uint32_t rank = __shfl_sync(0xffffffffu, cluster_rank(), 0);
   const bool leader = rank == 0;
   const AbortCtx ab{cta_abort, p.status};
   cg::cluster_group cluster = cg::this_cluster();
@@ -188,7 +188,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int tiles_m = (p.M + 2 * k2BM - 1) / (2 * k2BM);
   const int tiles_n = (p.N + k2BN - 1) / k2BN;
   const int ksplit = p.ksplit;
-  const int total_tiles = tiles_m * tiles_n * ksplit;      // work items
+  const int tiles_per_batch = tiles_m * tiles_n;
+  const int total_tiles = tiles_per_batch * p.batch * ksplit;      // work items
   const int num_kb = (p.K + k2BK - 1) / k2BK;
   const int pairs = gridDim.x / 2;
   const int pair = blockIdx.x / 2;
@@ -208,7 +209,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tma_prefetch_desc(&tmB);
   }
   if (warp == 1) {
-    tmem_alloc2(tmem_slot, ACC * k2BN);
+    tmem_alloc2(tmem_slot, 2 * k2BN);
     tmem_relinquish2();
   }
   tc_fence_before_sync();
@@ -217,11 +218,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_after_sync();
   // the MMA of the leader addresses the accumulator in both CTAs by the leader's allocation
   const uint32_t my_alloc = *tmem_slot;
-  const uint32_t tmem_base = leader ? my_alloc : ld_remote_u32(map_to_rank(smem_u32(tmem_slot), 0));
-  if (p.debug && threadIdx.x == 0 && pair == 0) {
-    p.debug[rank * 2] = static_cast<int>(my_alloc);
-    p.debug[rank * 2 + 1] = static_cast<int>(tmem_base);
-  }
+  const uint32_t tmem_base =
+      __shfl_sync(0xffffffffu, leader ? my_alloc : ld_remote_u32(map_to_rank(smem_u32(tmem_slot), 0)), 0);
 
   // k-block range [kb0, kb1) of a work item
   auto k_range = [&](int item, int& kb0, int& kb1) {
@@ -229,8 +227,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     kb0 = static_cast<int>(static_cast<long long>(ks) * num_kb / ksplit);
     kb1 = static_cast<int>(static_cast<long long>(ks + 1) * num_kb / ksplit);
   };
-  auto tile_coords = [&](int item, int& m_blk, int& n_blk) {
-    const int tile = item / ksplit;
+  auto tile_coords = [&](int item, int& b, int& m_blk, int& n_blk) {
+    const int all = item / ksplit;
+    b = all / tiles_per_batch;
+    const int tile = all - b * tiles_per_batch;
     const int group_sz = 4 * tiles_n;            // groups of 4 m-tiles share B tiles in L2
     const int g = tile / group_sz;
     const int first_m = g * 4;
@@ -247,8 +247,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
-        int m_blk, n_blk;
-        tile_coords(tile, m_blk, n_blk);
+        int b, m_blk, n_blk;
+        tile_coords(tile, b, m_blk, n_blk);
         const int m0 = m_blk * 2 * k2BM + static_cast<int>(rank) * k2BM;
         const int n0 = n_blk * k2BN + static_cast<int>(rank) * (k2BN / 2);
         int kb0, kb1;
@@ -263,15 +263,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           const int k0 = kb * k2BK;
           if (A_MN) {
 #pragma unroll
-            for (int j = 0; j < k2BM / 64; ++j) tma_load_3d_pair(a_dst + j * 8192, &tmA, bar, m0 + 64 * j, k0, 0);
+            for (int j = 0; j < k2BM / 64; ++j) tma_load_3d_pair(a_dst + j * 8192, &tmA, bar, m0 + 64 * j, k0, b);
           } else {
-            tma_load_3d_pair(a_dst, &tmA, bar, k0, m0, 0);
+            tma_load_3d_pair(a_dst, &tmA, bar, k0, m0, b);
           }
           if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < k2BN / 128; ++j) tma_load_3d_pair(b_dst + j * 8192, &tmB, bar, n0 + 64 * j, k0, 0);
+            for (int j = 0; j < k2BN / 128; ++j) tma_load_3d_pair(b_dst + j * 8192, &tmB, bar, n0 + 64 * j, k0, b);
           } else {
-            tma_load_3d_pair(b_dst, &tmB, bar, k0, n0, 0);
+            tma_load_3d_pair(b_dst, &tmB, bar, k0, n0, b);
           }
           if (++s == k2Stages) { s = 0; ph ^= 1; }
         }
@@ -279,40 +279,40 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      if (leader) {
-        // ---------------------------------------------------------------- MMA issuer (leader CTA)
-        constexpr uint32_t idesc = umma_idesc_bf16(2 * k2BM, k2BN, A_MN, B_MN);
-        int s = 0;
-        uint32_t ph = 0;
-        int it = 0;
-        bool ok = true;
-        for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
-          const int acc = ACC == 2 ? (it & 1) : 0;
-          const uint32_t acc_ph = ACC == 2 ? ((it >> 1) & 1) : (it & 1);
-          if (!mbar_wait_cluster(&tempty_bar[acc], acc_ph ^ 1, ab)) { ok = false; break; }
+    if (leader) {
+      // ------------------------------------------------------------------ MMA issuer (leader CTA, whole warp)
+      const uint32_t idesc = p.fp16 ? umma_idesc_f16(2 * k2BM, k2BN, A_MN, B_MN)
+                                    : umma_idesc_bf16(2 * k2BM, k2BN, A_MN, B_MN);
+      const uint32_t lead = elect_one();
+      const uint64_t a_desc = umma_smem_desc(smem_u32(smem_a), A_MN ? 8192 : 16, 1024);
+      const uint64_t b_desc = umma_smem_desc(smem_u32(smem_b), B_MN ? 8192 : 16, 1024);
+      int s = 0;
+      uint32_t ph = 0;
+      int it = 0;
+      bool ok = true;
+      for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
+        const int acc = it & 1;
+        const uint32_t acc_ph = (it >> 1) & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait_cluster(&tempty_bar[acc], acc_ph ^ 1, ab))) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + acc * k2BN;
+        int kb0, kb1;
+        k_range(tile, kb0, kb1);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait_warp(&full_bar[s], ph, ab)) { ok = false; break; }      // both CTAs' halves have landed
           tc_fence_after_sync();
-          const uint32_t d_tmem = tmem_base + acc * k2BN;
-          int kb0, kb1;
-          k_range(tile, kb0, kb1);
-          for (int kb = kb0; kb < kb1; ++kb) {
-            if (!mbar_wait(&full_bar[s], ph, ab)) { ok = false; break; }      // both CTAs' halves have landed
-            tc_fence_after_sync();
-            const uint32_t a_addr = smem_u32(smem_a + s * k2ABytes);
-            const uint32_t b_addr = smem_u32(smem_b + s * k2BBytes);
+          const uint64_t ad = a_desc + s * (k2ABytes >> 4), bd = b_desc + s * (k2BBytes >> 4);
+          if (lead) {
 #pragma unroll
-            for (int kk = 0; kk < k2BK / 16; ++kk) {
-              const uint64_t adesc = A_MN ? umma_smem_desc(a_addr + kk * 2048, 8192, 1024)
-                                          : umma_smem_desc(a_addr + kk * 32, 16, 1024);
-              const uint64_t bdesc = B_MN ? umma_smem_desc(b_addr + kk * 2048, 8192, 1024)
-                                          : umma_smem_desc(b_addr + kk * 32, 16, 1024);
-              umma2_bf16(d_tmem, adesc, bdesc, idesc, ((kb - kb0) | kk) != 0);
-            }
+            for (int kk = 0; kk < k2BK / 16; ++kk)
+              umma2_bf16(d_tmem, ad + kk * (A_MN ? 128 : 2), bd + kk * (B_MN ? 128 : 2), idesc, ((kb - kb0) | kk) != 0);
             umma2_commit_pair(&empty_bar[s]);
-            if (++s == k2Stages) { s = 0; ph ^= 1; }
           }
-          if (ok) umma2_commit_pair(&tfull_bar[acc]);
+          __syncwarp();
+          if (++s == k2Stages) { s = 0; ph ^= 1; }
         }
+        if (ok && lead) umma2_commit_pair(&tfull_bar[acc]);
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -326,10 +326,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const uint32_t tempty_leader1 = map_to_rank(smem_u32(&tempty_bar[1]), 0);
     const int sw = lane & 7;
     for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++it) {
-      int m_blk, n_blk;
-      tile_coords(tile, m_blk, n_blk);
-      const int acc = ACC == 2 ? (it & 1) : 0;
-      const uint32_t acc_ph = ACC == 2 ? ((it >> 1) & 1) : (it & 1);
+      int b, m_blk, n_blk;
+      tile_coords(tile, b, m_blk, n_blk);
+      const int acc = it & 1;
+      const uint32_t acc_ph = (it >> 1) & 1;
       if (!mbar_wait_cluster(&tfull_bar[acc], acc_ph, ab)) { ok = false; break; }
       tc_fence_after_sync();
       const int row0 = m_blk * 2 * k2BM + static_cast<int>(rank) * k2BM + q * 32;
@@ -347,10 +347,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
         if (p.bias) {
-          const __nv_bfloat16* bias = static_cast<const __nv_bfloat16*>(p.bias);
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (col0 + j < p.N) v[j] += __bfloat162float(bias[col0 + j]);
+            if (col0 + j < p.N) v[j] += load_16(p.bias, col0 + j, p.fp16);
         }
         uint8_t* rowp = stage_base + lane * 128;
         if (p.out_fp32) {
@@ -363,8 +362,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (p.accumulate) tma_reduce_add_3d_2(&tmC, stage_base, col0, row0, 0);
-            else tma_store_3d_2(&tmC, stage_base, col0, row0, 0);
+            if (p.accumulate) tma_reduce_add_3d_2(&tmC, stage_base, col0, row0, b);
+            else tma_store_3d_2(&tmC, stage_base, col0, row0, b);
             tma_store_commit();
           }
           ++nbuf;
@@ -377,10 +376,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             uint4 o;
-            o.x = pack_bf16x2(v[8 * j], v[8 * j + 1]);
-            o.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
-            o.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
-            o.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
+            o.x = pack_16x2(v[8 * j], v[8 * j + 1], p.fp16);
+            o.y = pack_16x2(v[8 * j + 2], v[8 * j + 3], p.fp16);
+            o.z = pack_16x2(v[8 * j + 4], v[8 * j + 5], p.fp16);
+            o.w = pack_16x2(v[8 * j + 6], v[8 * j + 7], p.fp16);
             *reinterpret_cast<uint4*>(rowp + (((half * 4 + j) ^ sw) << 4)) = o;
           }
           const bool last = (c + 32 >= k2BN) || (n0 + c + 32 >= p.N);
@@ -388,7 +387,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              tma_store_3d_2(&tmC, stage_base, col0 - half * 32, row0, 0);
+              tma_store_3d_2(&tmC, stage_base, col0 - half * 32, row0, b);
               tma_store_commit();
             }
             ++nbuf;
@@ -409,7 +408,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster.sync();          // the partner no longer reads this CTA's shared memory or signals its barriers
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc2(my_alloc, ACC * k2BN);
+    tmem_dealloc2(my_alloc, 2 * k2BN);
   }
 }
 
@@ -422,10 +421,10 @@ static int g_pair_splitk_auto = 1;
 // 1 (default): accumulating fp32 GEMMs choose a split-K factor by themselves; 0: never split.
 MSB_EXPORT void msb_gemm_pair_set_splitk(int enabled) { g_pair_splitk_auto = enabled ? 1 : 0; }
 
-template <bool A_MN, bool B_MN, int ACC>
+template <bool A_MN, bool B_MN>
 static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const Gemm2Params& p,
                         cudaStream_t stream) {
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, ACC>;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
     MSB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, k2SmemBytes));
@@ -451,7 +450,7 @@ static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CU
     if (n <= 0) { set_last_error("gemm_pair: no 2-CTA cluster of this kernel can be resident"); return kCudaError; }
     max_pairs = n;
   }
-  const int tiles = ((p.M + 255) / 256) * ((p.N + 255) / 256);
+  const int tiles = ((p.M + 255) / 256) * ((p.N + 255) / 256) * p.batch;
   Gemm2Params q = p;
   q.ksplit = 1;
   if (p.ksplit == 0 && p.accumulate && p.out_fp32 && !p.bias && g_pair_splitk_auto) {
@@ -480,43 +479,46 @@ static int launch_gemm2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CU
   return kOk;
 }
 
-// C (+)= alpha * A x B^T (+ bias) with CTA pairs.  Same operand conventions as msb_gemm_bf16 (no batch).  The output
-// must satisfy the TMA rules (16-byte aligned base and row pitch); bf16 accumulation is not supported.
-// acc_buffers: 1 or 2 accumulators in tensor memory.  debug: optional int[4] (device) receiving tensor-memory
-// addresses.
-MSB_EXPORT int msb_gemm_bf16_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
-                                  int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int out_fp32,
-                                  int accumulate, float alpha, int acc_buffers, int* debug, void* stream_) {
-  if (M <= 0 || N <= 0 || K <= 0) { set_last_error("gemm_pair: empty problem"); return kBadArg; }
-  if ((lda % 8) || (ldb % 8)) { set_last_error("gemm_pair: operand pitches must be multiples of 8"); return kBadArg; }
-  const int es = out_fp32 ? 4 : 2;
-  if ((reinterpret_cast<uintptr_t>(C) & 15) || ((ldc * es) & 15) || (accumulate && !out_fp32)) {
-    set_last_error("gemm_pair: output needs a 16-byte aligned base and pitch, and fp32 when accumulating");
+// C[b] (+)= alpha * A[b] x B[b]^T (+ bias) with CTA pairs.  Same operand conventions as msb_gemm_bf16.  The output must
+// satisfy the TMA rules (16-byte aligned base, row pitch and batch stride); 16-bit accumulation is not supported.
+// fp16: operands (and bias, and a 16-bit output) are fp16 instead of bf16.
+MSB_EXPORT int msb_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch,
+                             int a_mn, int b_mn, long long lda, long long ldb, long long ldc, long long a_bs,
+                             long long b_bs, long long c_bs, int out_fp32, int accumulate, float alpha, int fp16,
+                             void* stream_) {
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) { set_last_error("gemm_pair: empty problem"); return kBadArg; }
+  if ((lda % 8) || (ldb % 8) || (batch > 1 && ((a_bs % 8) || (b_bs % 8)))) {
+    set_last_error("gemm_pair: operand pitches and batch strides must be multiples of 8");
     return kBadArg;
   }
-  if (acc_buffers != 1 && acc_buffers != 2) { set_last_error("gemm_pair: acc_buffers must be 1 or 2"); return kBadArg; }
+  const int es = out_fp32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(C) & 15) || ((ldc * es) & 15) || (batch > 1 && ((c_bs * es) & 15)) ||
+      (accumulate && !out_fp32)) {
+    set_last_error("gemm_pair: output needs a 16-byte aligned base, pitch and batch stride, and fp32 when accumulating");
+    return kBadArg;
+  }
   Gemm2Params p = {};
-  p.bias = bias; p.status = status_ptr(); p.debug = debug;
+  p.bias = bias; p.status = status_ptr();
   if (!p.status) { set_last_error("gemm_pair: no status word"); return kCudaError; }
-  p.M = M; p.N = N; p.K = K; p.out_fp32 = out_fp32; p.accumulate = accumulate; p.alpha = alpha;
+  p.M = M; p.N = N; p.K = K; p.batch = batch; p.out_fp32 = out_fp32; p.accumulate = accumulate; p.alpha = alpha;
+  p.fp16 = fp16;
+  const uint64_t as = batch > 1 ? (uint64_t)a_bs * 2 : (uint64_t)lda * 2 * (a_mn ? K : M);
+  const uint64_t bs = batch > 1 ? (uint64_t)b_bs * 2 : (uint64_t)ldb * 2 * (b_mn ? K : N);
+  const uint64_t cs = batch > 1 ? (uint64_t)c_bs * es : (uint64_t)ldc * es * M;
   CUtensorMap tmA, tmB, tmC;
   int rc;
-  if (a_mn) rc = encode_tmap_3d(&tmA, A, 2, M, K, 1, lda * 2, (uint64_t)lda * 2 * K, 64, 64, 1);
-  else      rc = encode_tmap_3d(&tmA, A, 2, K, M, 1, lda * 2, (uint64_t)lda * 2 * M, 64, k2BM, 1);
+  if (a_mn) rc = encode_tmap_3d(&tmA, A, 2, M, K, batch, lda * 2, as, 64, 64, 1);
+  else      rc = encode_tmap_3d(&tmA, A, 2, K, M, batch, lda * 2, as, 64, k2BM, 1);
   if (rc) return rc;
-  if (b_mn) rc = encode_tmap_3d(&tmB, B, 2, N, K, 1, ldb * 2, (uint64_t)ldb * 2 * K, 64, 64, 1);
-  else      rc = encode_tmap_3d(&tmB, B, 2, K, N, 1, ldb * 2, (uint64_t)ldb * 2 * N, 64, k2BN / 2, 1);
+  if (b_mn) rc = encode_tmap_3d(&tmB, B, 2, N, K, batch, ldb * 2, bs, 64, 64, 1);
+  else      rc = encode_tmap_3d(&tmB, B, 2, K, N, batch, ldb * 2, bs, 64, k2BN / 2, 1);
   if (rc) return rc;
-  if ((rc = encode_tmap_3d(&tmC, C, es, N, M, 1, (uint64_t)ldc * es, (uint64_t)ldc * es * M, 128 / es, 32, 1))) return rc;
+  if ((rc = encode_tmap_3d(&tmC, C, es, N, M, batch, (uint64_t)ldc * es, cs, 128 / es, 32, 1))) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-#define MSB_PAIR(ACC_)                                                                     \
-  if (a_mn) {                                                                              \
-    if (b_mn) return launch_gemm2<true, true, ACC_>(tmA, tmB, tmC, p, stream);             \
-    return launch_gemm2<true, false, ACC_>(tmA, tmB, tmC, p, stream);                      \
-  } else {                                                                                 \
-    if (b_mn) return launch_gemm2<false, true, ACC_>(tmA, tmB, tmC, p, stream);            \
-    return launch_gemm2<false, false, ACC_>(tmA, tmB, tmC, p, stream);                     \
+  if (a_mn) {
+    if (b_mn) return launch_gemm2<true, true>(tmA, tmB, tmC, p, stream);
+    return launch_gemm2<true, false>(tmA, tmB, tmC, p, stream);
   }
-  if (acc_buffers == 2) { MSB_PAIR(2) } else { MSB_PAIR(1) }
-#undef MSB_PAIR
+  if (b_mn) return launch_gemm2<false, true>(tmA, tmB, tmC, p, stream);
+  return launch_gemm2<false, false>(tmA, tmB, tmC, p, stream);
 }

@@ -119,7 +119,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* issued_cnt = cta_abort + 1;    // k-blocks whose loads were issued
   volatile int* consumed_cnt = cta_abort + 2;  // k-blocks whose loads were observed complete
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   const AbortCtx ab{cta_abort, p.status};
 
@@ -152,7 +152,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   auto tile_coords = [&](int tile, int& b, int& m_blk, int& n_blk) {
     b = tile / tiles_per_batch;
@@ -229,42 +229,41 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
-      const uint32_t idesc = p.fp16 ? umma_idesc_f16(kBM, BN, A_MN, B_MN) : umma_idesc_bf16(kBM, BN, A_MN, B_MN);
-      int s = 0;
-      uint32_t ph = 0;
-      int it = 0;
-      int consumed = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-        const int acc = it & 1;
-        const uint32_t acc_ph = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_ph ^ 1, ab)) { ok = false; break; }
+    // -------------------------------------------------------------------- MMA issuer (whole warp, one elected lane)
+    const uint32_t idesc = p.fp16 ? umma_idesc_f16(kBM, BN, A_MN, B_MN) : umma_idesc_bf16(kBM, BN, A_MN, B_MN);
+    const uint32_t lead = elect_one();
+    // K-major: step 16 elements (32 B) inside the 128 B swizzle row.
+    // MN-major: step 16 k-rows of 128 B (2048 B); 64-wide M/N groups are 8192 B apart.
+    const uint64_t a_desc = umma_smem_desc(smem_u32(smem_a), A_MN ? 8192 : 16, 1024);
+    const uint64_t b_desc = umma_smem_desc(smem_u32(smem_b), B_MN ? 8192 : 16, 1024);
+    int s = 0;
+    uint32_t ph = 0;
+    int it = 0;
+    int consumed = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      const int acc = it & 1;
+      const uint32_t acc_ph = (it >> 1) & 1;
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_ph ^ 1, ab)) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&full_bar[s], ph, ab)) { ok = false; break; }
+        ++consumed;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full_bar[s], ph, ab)) { ok = false; break; }
-          ++consumed;
+        const uint64_t ad = a_desc + s * (Cfg::kABytes >> 4), bd = b_desc + s * (Cfg::kBBytes >> 4);
+        if (lead) {
           *consumed_cnt = consumed;
-          tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(smem_a + s * Cfg::kABytes);
-          const uint32_t b_addr = smem_u32(smem_b + s * Cfg::kBBytes);
 #pragma unroll
-          for (int kk = 0; kk < kBK / 16; ++kk) {
-            // K-major: step 16 elements (32 B) inside the 128 B swizzle row.
-            // MN-major: step 16 k-rows of 128 B (2048 B); 64-wide M/N groups are 8192 B apart.
-            const uint64_t adesc = A_MN ? umma_smem_desc(a_addr + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(a_addr + kk * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc(b_addr + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(b_addr + kk * 32, 16, 1024);
-            umma_bf16(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0);
-          }
+          for (int kk = 0; kk < kBK / 16; ++kk)
+            umma_bf16(d_tmem, ad + kk * (A_MN ? 128 : 2), bd + kk * (B_MN ? 128 : 2), idesc, (kb | kk) != 0);
           umma_commit(&empty_bar[s]);  // stage reusable once these MMAs retire
-          if (++s == kStages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(&tfull_bar[acc]);
+        __syncwarp();
+        if (++s == kStages) { s = 0; ph ^= 1; }
       }
+      if (ok && lead) umma_commit(&tfull_bar[acc]);
+      __syncwarp();
     }
     __syncwarp();
   } else if (warp < 6) {

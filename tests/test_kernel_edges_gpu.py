@@ -216,6 +216,27 @@ def test_fill_scalars(K):
     assert torch.equal(h.cpu(), torch.tensor([0, 0, 0.1, 1e-8, 3, 0, 0, 0]))
 
 
+# ------------------------------------------------------------------------------------------------ GEMM
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,Kd", [(1032, 776, 200), (1280, 2560, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_cta_pair_batched(K, a_mn, b_mn, M, N, Kd, dtype):
+    """Batched problems on CTA pairs, both element types, ragged tiles, accumulation."""
+    batch = 8
+    mk = lambda r, c, t: (torch.randn(batch, *((c, r) if t else (r, c)), device=DEV) / math.sqrt(Kd)).to(dtype)  # noqa: E731
+    a, b = mk(M, Kd, a_mn), mk(N, Kd, b_mn)
+    out = torch.empty(batch, M, N, device=DEV, dtype=dtype)
+    assert K._pair_gemm_ok(M, N, Kd, batch, out, out[0], False, 0)
+    ad = a.double().transpose(-1, -2) if a_mn else a.double()
+    bd = b.double().transpose(-1, -2) if b_mn else b.double()
+    ref = ad @ bd.transpose(-1, -2)
+    _near(K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out), ref, 2, dtype)
+    acc = torch.ones(ref.shape, device=DEV)
+    K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=acc, accumulate=True)
+    _near(acc, ref + 1, 256, torch.float32)
+    _status_ok()
+
+
 # ------------------------------------------------------------------------------------------------ convolution
 @pytest.mark.parametrize("N,C,H,W,Cout,k,stride", [(1, 64, 7, 7, 64, 3, 1), (3, 64, 13, 9, 256, 1, 1),
                                                   (2, 128, 15, 15, 128, 3, 2), (5, 64, 3, 5, 320, 1, 1)])
