@@ -19,6 +19,7 @@
 // full/empty mbarriers; tcgen05.commit releases a stage when the MMAs that read it retire.
 #include "host_common.h"
 #include "ptx.cuh"
+#include "gemm_small.cuh"
 
 namespace msb {
 
@@ -611,11 +612,27 @@ static int gemm_16(const void* A, const void* B, void* C, const void* bias, int 
     return kCudaError;
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const int bn = pick_bn(M, N, batch, bn_hint);
+  const int split = (bn_hint == 0 && !(accumulate && !out_fp32)) ? gemm_small_split(M, N, K, batch) : 0;
+  const int bn = split ? kGsBN : pick_bn(M, N, batch, bn_hint);
   CUtensorMap tmA, tmB;
   if (int rc = encode_operands(&tmA, &tmB, A, B, M, N, K, batch, a_mn, b_mn, lda, ldb, a_batch_stride,
                                b_batch_stride, bn))
     return rc;
+  if (split) {
+    const int es = out_fp32 ? 4 : 2;
+    GemmSmallParams q = {};
+    q.C = C; q.bias = bias; q.status = status; q.c_batch_stride = c_batch_stride; q.ldc = ldc;
+    q.M = M; q.N = N; q.K = K; q.split = split;
+    q.tiles_m = (M + kGsBM - 1) / kGsBM; q.tiles_n = (N + kGsBN - 1) / kGsBN;
+    q.out_fp32 = out_fp32; q.accumulate = accumulate; q.fp16 = fp16; q.alpha = alpha;
+    q.vec_ok = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ((ldc * es) & 15) == 0 && ((c_batch_stride * es) & 15) == 0;
+    if (a_mn) {
+      if (b_mn) return launch_gemm_small<true, true>(tmA, tmB, q, batch, stream);
+      return launch_gemm_small<true, false>(tmA, tmB, q, batch, stream);
+    }
+    if (b_mn) return launch_gemm_small<false, true>(tmA, tmB, q, batch, stream);
+    return launch_gemm_small<false, false>(tmA, tmB, q, batch, stream);
+  }
   GemmParams p = {};
   p.C = C; p.bias = bias; p.status = status; p.c_batch_stride = c_batch_stride;
   p.M = M; p.N = N; p.K = K; p.batch = batch; p.ldc = static_cast<int>(ldc);

@@ -217,6 +217,28 @@ def test_fill_scalars(K):
 
 
 # ------------------------------------------------------------------------------------------------ GEMM
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,Kd,batch", [(8, 8, 8, 1), (24, 4096, 4096, 1), (136, 72, 328, 1), (128, 64, 520, 3),
+                                          (1, 200, 2048, 1), (300, 512, 1408, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_with_few_tiles(K, a_mn, b_mn, M, N, Kd, batch, dtype):
+    """Split over clusters of 1 to 8 CTAs, ragged M / N / K, bias, fp32 accumulation into an existing output."""
+    if a_mn and M % 8:
+        pytest.skip("a stored [K, M] needs a row pitch of whole 16 bytes")
+    mk = lambda r, c, t: (torch.randn(*((batch,) if batch > 1 else ()), *((c, r) if t else (r, c)), device=DEV) /  # noqa: E731
+                          math.sqrt(Kd)).to(dtype)
+    a, b = mk(M, Kd, a_mn), mk(N, Kd, b_mn)
+    bias = torch.randn(N, device=DEV).to(dtype)
+    ad = a.double().transpose(-1, -2) if a_mn else a.double()
+    bd = b.double().transpose(-1, -2) if b_mn else b.double()
+    ref = ad @ bd.transpose(-1, -2)
+    _near(K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=2.0), 2 * ref + bias.double(), 2, dtype)
+    out = torch.ones(ref.shape, device=DEV)
+    K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=True)
+    _near(out, ref + 1, 256, torch.float32)                     # fp32 sums of up to 4096 products in another order
+    _status_ok()
+
+
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("M,N,Kd", [(1032, 776, 200), (1280, 2560, 72)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
