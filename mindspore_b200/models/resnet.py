@@ -13,7 +13,7 @@ import torch
 from .. import nn
 from ..common.initializer import HeNormal, initializer
 from ..common.parameter import Parameter
-from ..ops import conv_kernel
+from ..ops import conv_kernel, fused
 from ..ops.primitive import _wrap_out
 
 
@@ -32,14 +32,15 @@ class ConvBnAct(nn.Cell):
 
     def construct(self, x, residual=None):
         w = self.conv.weight
-        if self.training and x.is_cuda and x.dtype == torch.bfloat16 and conv_kernel.available() \
-                and w.shape[0] % 64 == 0:
-            bn = self.bn
-            y = conv_kernel.conv_bn_act(x.as_subclass(torch.Tensor), w, bn.gamma, bn.beta,
-                                        bn.moving_mean.detach().as_subclass(torch.Tensor),
-                                        bn.moving_variance.detach().as_subclass(torch.Tensor), self.stride, self.pad,
-                                        self.relu, residual, bn.eps, bn.momentum)
-            return _wrap_out(y)
+        with fused.quiet():
+            if self.training and x.is_cuda and x.dtype == torch.bfloat16 and conv_kernel.available() \
+                    and w.shape[0] % 64 == 0:
+                bn = self.bn
+                y = conv_kernel.conv_bn_act(x.as_subclass(torch.Tensor), w, bn.gamma, bn.beta,
+                                            bn.moving_mean.detach().as_subclass(torch.Tensor),
+                                            bn.moving_variance.detach().as_subclass(torch.Tensor), self.stride, self.pad,
+                                            self.relu, residual, bn.eps, bn.momentum)
+                return _wrap_out(y)
         y = self.bn(self.conv(x))
         if residual is not None:
             y = y + residual

@@ -12,6 +12,8 @@ import math
 import torch
 import torch.nn.functional as F
 
+from .fused import quiet
+
 _impl = None
 
 
@@ -41,6 +43,8 @@ def reference_attention(q, k, v, causal=True, scale=None):
 
 def flash_attention(q, k, v, causal=True, scale=None):
     impl = _kernel_impl()
-    if impl and impl.supports(q, k, v) and (scale is None or scale > 0):      # the kernel's running maximum needs that
-        return impl.flash_attention(q, k, v, causal, scale)
+    if impl:
+        with quiet():
+            if impl.supports(q, k, v) and (scale is None or scale > 0):      # the kernel's running maximum needs that
+                return impl.flash_attention(q, k, v, causal, scale)
     return reference_attention(q, k, v, causal, scale)

@@ -16,6 +16,7 @@ import torch
 
 from .. import _native
 from . import kernels as K
+from .fused import _quietly, quiet
 from .kernels import _count, _p, _stream
 
 _P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
@@ -149,6 +150,7 @@ class _ConvFn(torch.autograd.Function):
         return y, None
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy, _dstats):
         x, w = ctx.saved_tensors
         stride, pad_h, pad_w, ho, wo = ctx.geom
@@ -249,6 +251,7 @@ class _BnActFn(torch.autograd.Function):
         return y
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         x, y, g, mean, rstd = ctx.saved_tensors
         n, c, h, w = x.shape
@@ -282,10 +285,11 @@ def conv_bn_act(x, w, gamma, beta, moving_mean, moving_var, stride=1, pad=0, rel
                 momentum=0.9):
     """Training-mode Conv2d -> BatchNorm2d -> (+ residual) -> ReLU on the kernel path.  ``momentum`` is the weight
     of the old moving statistics (nn.BatchNorm2d convention)."""
-    wb = w if w.dtype == x.dtype else w.to(x.dtype)
-    _producer(wb, gamma, beta)
-    y, stats = _ConvFn.apply(x, wb, stride, pad, pad, True)
-    return _BnActFn.apply(y, stats, gamma, beta, residual, relu, eps, (moving_mean, moving_var, momentum))
+    with quiet():
+        wb = w if w.dtype == x.dtype else w.to(x.dtype)
+        _producer(wb, gamma, beta)
+        y, stats = _ConvFn.apply(x, wb, stride, pad, pad, True)
+        return _BnActFn.apply(y, stats, gamma, beta, residual, relu, eps, (moving_mean, moving_var, momentum))
 
 
 def bn_act_inference(x, gamma, beta, moving_mean, moving_var, relu=True, residual=None, eps=1e-5):
@@ -323,6 +327,7 @@ class _MaxPool3x3s2Fn(torch.autograd.Function):
         return y
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         (idx,) = ctx.saved_tensors
         n, c, h, w = ctx.shape
@@ -345,6 +350,7 @@ class _GlobalAvgPoolFn(torch.autograd.Function):
         return y
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         n, c, h, w = ctx.shape
         dx = _empty(n, c, h, w, dy.device, dy.dtype)

@@ -6,6 +6,7 @@ import torch
 
 from .. import _native
 from . import kernels as K
+from .fused import _quietly
 from .kernels import _count, _p, _stream
 
 _P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
@@ -114,6 +115,7 @@ class _FlashFn(torch.autograd.Function):
         return o
 
     @staticmethod
+    @_quietly
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
         dq, dk, dv = bwd(do, q, k, v, o, lse, ctx.causal, ctx.scale)

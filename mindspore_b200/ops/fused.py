@@ -7,12 +7,67 @@ has one, which folds micro-batch gradient accumulation into the wgrad GEMM epilo
 """
 from __future__ import annotations
 
+import contextlib
+import functools
 import math
 
 import torch
 import torch.nn.functional as F
 
+from ..common.parameter import Parameter
+from ..common.tensor import Tensor, _sharded_mode
 from . import kernels as K
+from . import primitive as _primitive
+
+
+_KNOWN_TYPES = (torch.Tensor, Tensor, Parameter)
+
+
+def quiet():
+    """Attribute reads and method calls on a ``Tensor`` / ``Parameter`` go through its ``__torch_function__``: 3 to 9 us
+    each, where a plain tensor takes 0.1, and a kernel wrapper makes dozens of them.  Code in this context reads the
+    tensors as what they are.  A trace sees every call as before, and so does the sharded dispatcher."""
+    if _primitive._trace_hook is not None or _sharded_mode():
+        return contextlib.nullcontext()
+    return torch._C.DisableTorchFunctionSubclass()
+
+
+def known(*tensors):
+    """Whether none of the tensors is of a class whose operators mean something else (a stand-in of a pipeline)."""
+    return all(type(t) in _KNOWN_TYPES for t in tensors)
+
+
+def _quietly(fn):
+    """``fn`` (a backward) under ``quiet``."""
+    @functools.wraps(fn)
+    def run(*args):
+        with quiet():
+            return fn(*args)
+    return run
+
+
+def _typed(out, x):
+    """``out`` as a framework ``Tensor`` when ``x`` is one, as a new tensor like ``x`` is outside ``quiet``."""
+    return out.as_subclass(Tensor) if isinstance(x, Tensor) else out
+
+
+def known(*tensors):
+    """Whether none of the tensors is of a class whose operators mean something else (a stand-in of a pipeline)."""
+    return all(type(t) in _KNOWN_TYPES for t in tensors)
+
+
+def _quietly(fn):
+    """``fn`` (a backward) under ``quiet``."""
+    @functools.wraps(fn)
+    def run(*args):
+        with quiet():
+            return fn(*args)
+    return run
+
+
+def _typed(out, *inputs):
+    """``out`` as a framework ``Tensor`` when one of the inputs is one: what the calls in ``quiet`` no longer do."""
+    return out.as_subclass(Tensor) if any(isinstance(t, Tensor) for t in inputs) else out
 
 
 def _use_kernel(*tensors, fp16_ok=False):
@@ -56,6 +111,7 @@ class _LinearFn(torch.autograd.Function):
         return y.view(*x.shape[:-1], w.shape[0])
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
@@ -80,9 +136,10 @@ class _LinearFn(torch.autograd.Function):
 
 def linear(x, w, bias=None):
     """y = x @ w^T + bias with w stored [out, in]."""
-    if _use_kernel(x, w, bias, fp16_ok=True) and x.shape[-1] % 8 == 0 and w.shape[0] % 8 == 0:
-        _producer(w)
-        return _LinearFn.apply(x, w, bias)
+    with quiet():
+        if _use_kernel(x, w, bias, fp16_ok=True) and x.shape[-1] % 8 == 0 and w.shape[0] % 8 == 0:
+            _producer(w)
+            return _LinearFn.apply(x, w, bias)
     return F.linear(x, w, bias)
 
 
@@ -101,6 +158,7 @@ class _MatMulFn(torch.autograd.Function):
         return K.gemm(a, b, a_mn=ta, b_mn=not tb)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dc):
         a, b = ctx.saved_tensors
         ta, tb = ctx.ta, ctx.tb
@@ -127,11 +185,12 @@ class _MatMulFn(torch.autograd.Function):
 
 
 def matmul(a, b, transpose_a=False, transpose_b=False):
-    if _use_kernel(a, b, fp16_ok=True) and a.dim() == b.dim() and a.dim() in (2, 3) and a.is_contiguous() and b.is_contiguous() \
-            and all(s % 8 == 0 for s in a.shape[-2:]) and all(s % 8 == 0 for s in b.shape[-2:]):
-        if b.dim() == 2 and getattr(b, "main_grad", None) is not None:
-            _producer(b)
-        return _MatMulFn.apply(a, b, bool(transpose_a), bool(transpose_b))
+    with quiet():
+        if (_use_kernel(a, b, fp16_ok=True) and a.dim() == b.dim() and a.dim() in (2, 3) and a.is_contiguous()
+                and b.is_contiguous() and all(s % 8 == 0 for s in a.shape[-2:]) and all(s % 8 == 0 for s in b.shape[-2:])):
+            if b.dim() == 2 and getattr(b, "main_grad", None) is not None:
+                _producer(b)
+            return _MatMulFn.apply(a, b, bool(transpose_a), bool(transpose_b))
     aa = a.transpose(-1, -2) if transpose_a else a
     bb = b.transpose(-1, -2) if transpose_b else b
     return torch.matmul(aa, bb)
@@ -149,12 +208,13 @@ class _RmsNormFn(torch.autograd.Function):
         rstd_out = rstd.view_as(rstd)
         ctx.mark_non_differentiable(rstd_out)
         if residual is not None:
-            return y, xsum, rstd_out
+            return _typed(y, x), _typed(xsum, x), rstd_out
         dummy = x.new_empty(0)
         ctx.mark_non_differentiable(dummy)
-        return y, dummy, rstd_out
+        return _typed(y, x), dummy, rstd_out
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy, dxsum, _drstd):
         xsum, w, rstd = ctx.saved_tensors
         if dy is None:
@@ -173,11 +233,12 @@ class _RmsNormFn(torch.autograd.Function):
 def rms_norm(x, w, eps=1e-6, residual=None, with_rstd=False):
     """Returns (y, stream) where stream = x + residual (or x).  y = stream * rsqrt(mean(stream^2)+eps) * w.
     ``with_rstd`` appends the per-row reciprocal RMS (fp32, shape [..., 1])."""
-    if _use_kernel(x, w, residual, fp16_ok=True) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        _producer(w)
-        y, stream, rstd = _RmsNormFn.apply(x, w, eps, residual)
-        stream = stream if residual is not None else x
-        return (y, stream, rstd.reshape(*x.shape[:-1], 1)) if with_rstd else (y, stream)
+    with quiet():
+        if _use_kernel(x, w, residual, fp16_ok=True) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
+            _producer(w)
+            y, stream, rstd = _RmsNormFn.apply(x, w, eps, residual)
+            stream = stream if residual is not None else x
+            return (y, stream, rstd.reshape(*x.shape[:-1], 1)) if with_rstd else (y, stream)
     stream = x if residual is None else x + residual
     xf = stream.float()
     rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
@@ -191,9 +252,10 @@ class _LayerNormFn(torch.autograd.Function):
         y, mean, rstd = K.layernorm_fwd(x.contiguous(), w, b, eps)
         ctx.save_for_backward(x, w, mean, rstd)
         ctx.w_ref, ctx.b_ref = w, b
-        return y
+        return _typed(y, x)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         x, w, mean, rstd = ctx.saved_tensors
         mgw = getattr(ctx.w_ref, "main_grad", None)
@@ -210,11 +272,12 @@ class _LayerNormFn(torch.autograd.Function):
 
 
 def layer_norm(x, w, b, eps=1e-5):
-    if _use_kernel(x, w, b, fp16_ok=True) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        _producer(w)
-        if b is not None:
-            _producer(b)
-        return _LayerNormFn.apply(x, w, b, eps)
+    with quiet():
+        if _use_kernel(x, w, b, fp16_ok=True) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
+            _producer(w)
+            if b is not None:
+                _producer(b)
+            return _LayerNormFn.apply(x, w, b, eps)
     return F.layer_norm(x, (x.shape[-1],), w, b, eps)
 
 
@@ -226,6 +289,7 @@ class _SwiGLUFn(torch.autograd.Function):
         return K.swiglu_fwd(gu)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dout):
         (gu,) = ctx.saved_tensors
         return K.swiglu_bwd(gu, dout.contiguous())
@@ -233,8 +297,9 @@ class _SwiGLUFn(torch.autograd.Function):
 
 def swiglu(gu):
     """silu(gu[..., :F]) * gu[..., F:]"""
-    if _use_kernel(gu, fp16_ok=True) and gu.is_contiguous() and (gu.shape[-1] // 2) % 8 == 0:
-        return _SwiGLUFn.apply(gu)
+    with quiet():
+        if _use_kernel(gu, fp16_ok=True) and gu.is_contiguous() and (gu.shape[-1] // 2) % 8 == 0:
+            return _SwiGLUFn.apply(gu)
     f = gu.shape[-1] // 2
     return F.silu(gu[..., :f]) * gu[..., f:]
 
@@ -244,9 +309,10 @@ class _GeluFn(torch.autograd.Function):
     def forward(ctx, x, bias):
         ctx.save_for_backward(x, bias)
         ctx.b_ref = bias
-        return K.gelu_fwd(x, bias)
+        return _typed(K.gelu_fwd(x, bias), x)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         x, bias = ctx.saved_tensors
         dx = K.gelu_bwd(x, dy.contiguous(), bias)
@@ -257,8 +323,9 @@ class _GeluFn(torch.autograd.Function):
 
 
 def gelu_tanh(x, bias=None):
-    if _use_kernel(x, bias, fp16_ok=True) and x.is_contiguous() and x.shape[-1] % 8 == 0:
-        return _GeluFn.apply(x, bias)
+    with quiet():
+        if _use_kernel(x, bias, fp16_ok=True) and x.is_contiguous() and x.shape[-1] % 8 == 0:
+            return _GeluFn.apply(x, bias)
     return F.gelu(x if bias is None else x + bias, approximate="tanh")
 
 
@@ -268,9 +335,10 @@ class _RopeFn(torch.autograd.Function):
     def forward(ctx, x, cos, sin, heads, head_dim, seq):
         ctx.save_for_backward(cos, sin)
         ctx.meta = (heads, head_dim, seq)
-        return K.rope(x, cos, sin, heads, head_dim, seq)
+        return _typed(K.rope(x, cos, sin, heads, head_dim, seq), x)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dy):
         cos, sin = ctx.saved_tensors
         heads, head_dim, seq = ctx.meta
@@ -285,8 +353,9 @@ def rope_tables(seq, head_dim, theta=10000.0, device="cpu"):
 
 def rope(x, cos, sin, heads, head_dim, seq):
     """Rotate-half RoPE on x[..., seq, heads*head_dim] (token-major); cos/sin fp32 [seq, head_dim/2]."""
-    if _use_kernel(x, fp16_ok=True) and x.is_contiguous() and head_dim % 16 == 0:
-        return _RopeFn.apply(x, cos, sin, heads, head_dim, seq)
+    with quiet():
+        if _use_kernel(x, fp16_ok=True) and x.is_contiguous() and head_dim % 16 == 0:
+            return _RopeFn.apply(x, cos, sin, heads, head_dim, seq)
     shp = x.shape
     xv = x.reshape(-1, seq, heads, head_dim).float()
     c = cos[None, :, None, :]
@@ -309,6 +378,7 @@ class _SoftmaxCEFn(torch.autograd.Function):
         return loss
 
     @staticmethod
+    @_quietly
     def backward(ctx, dloss):
         logits, labels, stats, count = ctx.saved_tensors
         scale = dloss.float().reshape(1).contiguous()
@@ -319,8 +389,9 @@ class _SoftmaxCEFn(torch.autograd.Function):
 
 def softmax_cross_entropy(logits, labels, ignore_index=-100):
     """Mean token cross entropy.  logits [..., V] (bf16 or fp32, CUDA) and integer labels [...]."""
-    if logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.is_contiguous():
-        return _SoftmaxCEFn.apply(logits, labels, ignore_index)
+    with quiet():
+        if logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.is_contiguous():
+            return _SoftmaxCEFn.apply(logits, labels, ignore_index)
     return F.cross_entropy(logits.reshape(-1, logits.shape[-1]).float(), labels.reshape(-1).long(),
                            ignore_index=ignore_index)
 
@@ -336,6 +407,7 @@ class _EmbeddingFn(torch.autograd.Function):
         return K.embedding_fwd(table, ids32, vocab_start)
 
     @staticmethod
+    @_quietly
     def backward(ctx, dout):
         (ids32,) = ctx.saved_tensors
         t = ctx.t_ref
@@ -350,9 +422,10 @@ class _EmbeddingFn(torch.autograd.Function):
 
 
 def embedding(table, ids, vocab_start=0):
-    if _use_kernel(table) and table.shape[1] % 8 == 0:
-        _producer(table)
-        return _EmbeddingFn.apply(table, ids, vocab_start)
+    with quiet():
+        if _use_kernel(table) and table.shape[1] % 8 == 0:
+            _producer(table)
+            return _EmbeddingFn.apply(table, ids, vocab_start)
     idx = ids.long() - vocab_start
     mask = (idx >= 0) & (idx < table.shape[0])
     return F.embedding(idx.clamp(0, table.shape[0] - 1), table) * mask.unsqueeze(-1).to(table.dtype)
@@ -392,6 +465,7 @@ class _QkvRopeAttnFn(torch.autograd.Function):
         return o
 
     @staticmethod
+    @_quietly
     def backward(ctx, do):
         from . import flash_attn_kernel as FK
         qk, qkv, o, lse, cos, sin = ctx.saved_tensors
@@ -413,9 +487,10 @@ def qkv_rope_attention(qkv, cos, sin, batch, seq, heads, kv_heads, head_dim, cau
     from . import flash_attn_kernel as FK
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     hd, kd = heads * head_dim, kv_heads * head_dim
-    if (_use_kernel(qkv, fp16_ok=True) and qkv.is_contiguous() and head_dim == 128
-            and heads % kv_heads == 0 and scale > 0 and FK.available() and FK.has_strided_bwd()):
-        return _QkvRopeAttnFn.apply(qkv, cos, sin, batch, seq, heads, kv_heads, head_dim, bool(causal), float(scale))
+    with quiet():
+        if (_use_kernel(qkv, fp16_ok=True) and qkv.is_contiguous() and head_dim == 128
+                and heads % kv_heads == 0 and scale > 0 and FK.available() and FK.has_strided_bwd()):
+            return _QkvRopeAttnFn.apply(qkv, cos, sin, batch, seq, heads, kv_heads, head_dim, bool(causal), float(scale))
     qk = rope(qkv[:, :hd + kd].contiguous(), cos, sin, heads + kv_heads, head_dim, seq)
     q = qk[:, :hd].reshape(batch, seq, heads, head_dim)
     k = qk[:, hd:].reshape(batch, seq, kv_heads, head_dim)

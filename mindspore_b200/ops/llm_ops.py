@@ -18,6 +18,7 @@ The reference composes these from Split / Mul / SiLU / ApplyRotaryPosEmb / Flash
 """
 from __future__ import annotations
 
+import contextlib
 import math
 
 import torch
@@ -77,6 +78,7 @@ class RotaryFlashAttention(Primitive):
         g = self.groups
         h, hk = self.head_num // g, self.kv_head_num // g
         if g == 1:
-            return self._one(qkv, cos, sin, h, hk)
+            with fused.quiet() if fused.known(qkv, cos, sin) else contextlib.nullcontext():
+                return self._one(qkv, cos, sin, h, hk)
         blk = (h + 2 * hk) * self.head_dim
         return torch.cat([self._one(qkv[:, i * blk:(i + 1) * blk].contiguous(), cos, sin, h, hk) for i in range(g)], -1)

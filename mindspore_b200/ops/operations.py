@@ -10,6 +10,7 @@ yaml op definitions under mindspore/core/ops/ops_def/.
 """
 from __future__ import annotations
 
+import contextlib
 import math
 import numbers
 
@@ -1014,6 +1015,10 @@ class FlashAttentionScore(Primitive):
 
     def _run(self, query, key, value, real_shift=None, drop_mask=None, padding_mask=None, attn_mask=None,
              prefix=None, actual_seq_qlen=None, actual_seq_kvlen=None):
+        with fused.quiet() if fused.known(query, key, value) else contextlib.nullcontext():
+            return self._attend(query, key, value, attn_mask)
+
+    def _attend(self, query, key, value, attn_mask):
         causal = self.next_tokens == 0 or self.sparse_mode in (2, 3)
         lay = self.input_layout
         H = self.head_num
