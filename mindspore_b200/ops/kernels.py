@@ -208,7 +208,7 @@ def layernorm_bwd(dy, x, w, mean, rstd, dw_out=None, db_out=None, accumulate=Fal
     rc = _fn("msb_layernorm_bwd", x)(_p(dy), _p(x), _p(w), _p(mean), _p(rstd), _p(dx), _p(acc), _p(dw_out),
                                           _p(db_out), int(dw_out.dtype == f32), int(accumulate), rows, H, _stream())
     _native.check(rc, "layernorm_bwd")
-    _count(3)
+    _count(2)
     return dx, dw_out, db_out
 
 
