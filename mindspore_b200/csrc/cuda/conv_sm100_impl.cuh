@@ -10,7 +10,8 @@
 //   squares of the output in shared memory (flushed once per CTA) - the BatchNorm statistics come for free.
 // Weight gradient (WGRAD = true):  dW[co, tap, ci] = sum_pix dY[pix, co] * X[pix + offset(tap), ci]
 //   GEMM M = Cout, N = Cin, K = pixels; both operands are MN-major 4-D box loads (64 pixels x 64 channels), the
-//   k-loop runs over pixel tiles and is split across CTAs (fp32 atomic accumulation into dW).
+//   k-loop runs over pixel tiles and is split across CTAs (fp32 atomic accumulation into dW).  Whole blocks of 64 input
+//   channels make N run over (tap, ci) together - the order of a row of dW -, so a tile of several narrow taps reads dY once.
 //
 // The reference calls cudnnConvolutionForward / BackwardData / BackwardFilter
 // (plugin/device/gpu/kernel/nn/conv2d_gpu_kernel.h, conv2d_grad_input_gpu_kernel.h, conv2d_grad_filter_gpu_kernel.h)
@@ -42,6 +43,7 @@ struct ConvParams {
   int Cout, Cin;
   long long ldc;         // fwd: elements between output pixels; wgrad: elements between rows of dW
   int out_fp32, accumulate, ksplit;
+  int flat;              // wgrad: the columns of the GEMM run over (tap, ci); 0: over ci, one tap per tile
   // 1: output tiles go through swizzled shared memory and leave as TMA stores (wgrad: TMA reduce-adds); 0: per-thread
   // stores / atomics, for fp32 forward outputs, channel counts and pitches that the tensor map cannot describe
   int tma_out;
@@ -59,7 +61,8 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* t
 
 template <int BN>
 struct ConvCfg {
-  static constexpr int kStages = (BN == 256) ? 3 : 5;
+  static constexpr int kStages = (BN == 256) ? 3 : (BN == 192) ? 4 : (BN == 128) ? 5 : 7;
+  static constexpr int kTmemCols = (BN == 192) ? 512 : 2 * BN;      // a power of two
   static constexpr int kABytes = kConvBM * kConvBK * 2;
   static constexpr int kBBytes = BN * kConvBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
@@ -116,9 +119,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
   // GEMM tiling
   const int gemm_m = WGRAD ? p.Cout : 0;
   const int tiles_m = WGRAD ? (gemm_m + kConvBM - 1) / kConvBM : pix_tiles;
-  const int gemm_n = WGRAD ? p.Cin : p.Cout;
+  const int gemm_n = WGRAD ? (p.flat ? p.taps * p.Cin : p.Cin) : p.Cout;
   const int tiles_n = (gemm_n + BN - 1) / BN;
-  const int outer = WGRAD ? p.taps * p.ksplit : 1;
+  const int outer = WGRAD ? (p.flat ? 1 : p.taps) * p.ksplit : 1;
   const int total_tiles = tiles_m * tiles_n * outer;
   const int kb_total = WGRAD ? pix_tiles : p.taps * p.cin_blocks;
   const int kb_per = WGRAD ? (kb_total + p.ksplit - 1) / p.ksplit : kb_total;
@@ -143,7 +146,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
   if (want_stats)
     for (int i = threadIdx.x; i < 2 * p.Cout; i += kConvThreads) s_stats[i] = 0.f;
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 2 * BN);
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -191,10 +194,27 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
         const int nc0 = n_blk * BN;
         int n0 = 0, h0 = 0, w0 = 0;
         if (!WGRAD) pixel_origin(m_blk, n0, h0, w0);
-        const int tap_w = WGRAD ? o / p.ksplit : 0;
+        // wgrad: where each 64-column block of B comes from, and how many blocks there are; what lies beyond the matrix is
+        // not loaded (its rows and columns of the product are not stored either)
+        const CUtensorMap* bx[BN / 64];
+        int bc[BN / 64], bh[BN / 64], bw[BN / 64], a_blocks = 2, b_blocks = BN / 64;
+        if (WGRAD) {
+          a_blocks = min(2, (p.Cout - m_blk * kConvBM + 63) / 64);
+          b_blocks = min(BN / 64, (gemm_n - nc0 + 63) / 64);
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) {
+            const int col = min(nc0 + 64 * j, gemm_n - 1);
+            const int tap = p.flat ? col / p.Cin : o / p.ksplit;
+            bx[j] = maps[p.tap_map[tap]];
+            bc[j] = p.flat ? col - tap * p.Cin : col;
+            bh[j] = p.tap_dh[tap];
+            bw[j] = p.tap_dw[tap];
+          }
+        }
+        const int stage_bytes = WGRAD ? (a_blocks + b_blocks) * 8192 : Cfg::kStageBytes;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1, ab)) { ok = false; break; }
-          mbar_expect_tx(&full_bar[s], Cfg::kStageBytes);
+          mbar_expect_tx(&full_bar[s], stage_bytes);
           uint8_t* a_dst = smem_a + s * Cfg::kABytes;
           uint8_t* b_dst = smem_b + s * Cfg::kBBytes;
           if (WGRAD) {
@@ -202,12 +222,10 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
             const int m0 = m_blk * kConvBM;
 #pragma unroll
             for (int j = 0; j < kConvBM / 64; ++j)
-              tma_load_4d(a_dst + j * 8192, &tmO, &full_bar[s], m0 + 64 * j, w0, h0, n0);
-            const CUtensorMap* mx = maps[p.tap_map[tap_w]];
-            const int dh = p.tap_dh[tap_w], dw = p.tap_dw[tap_w];
+              if (j < a_blocks) tma_load_4d(a_dst + j * 8192, &tmO, &full_bar[s], m0 + 64 * j, w0, h0, n0);
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_4d(b_dst + j * 8192, mx, &full_bar[s], nc0 + 64 * j, w0 + dw, h0 + dh, n0);
+              if (j < b_blocks) tma_load_4d(b_dst + j * 8192, bx[j], &full_bar[s], bc[j], w0 + bw[j], h0 + bh[j], n0);
           } else {
             const int tap = kb / p.cin_blocks;
             const int cb = kb - tap * p.cin_blocks;
@@ -266,7 +284,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
     // Two groups of four warps take the tiles in turn, each on its own accumulator.  A 1x1 convolution of 256 channels
     // has about 2700 cycles per tile from HBM's side; one group with per-thread row stores needed four times that.
     // 64 x 56 x 56 pixels, 64 -> 256 and back: 64 -> 31 us each; weight gradients, whose tiles left as fp32 atomics of
-    // single elements: 88 -> 29 us (1x1, 256 columns) and 91 -> 62 us (128 columns).
+    // single elements: 88 -> 29 us (1x1, 256 columns).
     const int q = warp & 3, grp = (warp - 2) >> 2;
     int it = grp;
     bool ok = true;
@@ -460,7 +478,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 2 * BN);
+    tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -568,7 +586,9 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
   CUtensorMap maps[4], tmW;
   if (int rc = setup_input(maps, &p, x, N, H, W, Cin, ldx, R, S, stride, pad_h, pad_w, flip)) return rc;
   const long long pix_tiles = static_cast<long long>(p.tiles_w) * p.tiles_h * p.tiles_n;
-  const int bn = (Cout <= 128 || pix_tiles * ((Cout + 255) / 256) < sm_count()) ? 128 : 256;
+  // Up to 64 channels: half of a 128-column tile's weight rows, products and shared memory would be padding (64 x 56 x 56,
+  // 1x1 256 -> 64 and 3x3 64 -> 64, forward and data gradient: 172 -> 139 us).
+  const int bn = Cout <= 64 ? 64 : (Cout <= 128 || pix_tiles * ((Cout + 255) / 256) < sm_count()) ? 128 : 256;
   const long long K = static_cast<long long>(R) * S * Cin;
   if (int rc = encode_tmap_3d(&tmW, w, 2, K, Cout, 1, K * 2, K * 2 * Cout, 64, bn, 1)) return rc;
   // the output as TMA sees it: a warp's 32 rows are a sub-box of the tile's (all extents are powers of two)
@@ -585,6 +605,7 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
   if (tiles > 0x7fffffffLL) { set_last_error("conv_fwd: too many tiles"); return kTooLarge; }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (bn == 256) return launch_conv<256, false>(maps, tmW, tmY, p, (int)tiles, stream);
+  if (bn == 64) return launch_conv<64, false>(maps, tmW, tmY, p, (int)tiles, stream);
   return launch_conv<128, false>(maps, tmW, tmY, p, (int)tiles, stream);
 }
 
@@ -611,8 +632,19 @@ MSB_EXPORT int MSB_FN(msb_conv_wgrad)(const void* x, const void* dy, float* dw, 
   const uint64_t dims[4] = {(uint64_t)Cout, (uint64_t)Wo, (uint64_t)Ho, (uint64_t)N};
   const uint64_t st[3] = {(uint64_t)(ldy * 2), (uint64_t)(Wo * ldy * 2), (uint64_t)((long long)Ho * Wo * ldy * 2)};
   if (int rc = encode_tmap_4d(&tmDY, dy, dims, st, box)) return rc;
-  const int bn = Cin <= 128 ? 128 : 256;
-  const long long base_tiles = static_cast<long long>((Cout + kConvBM - 1) / kConvBM) * ((Cin + bn - 1) / bn) * p.taps;
+  // The feed of shared memory bounds a tile (an A block of 128 rows costs as much as 128 columns of B), so: the fewest
+  // tiles, and of the widths that give that count the narrowest.  64 x 56 x 56, 3x3 64 -> 64 and 1x1 64 -> 256 together, one
+  // tap per tile of 128 columns 122 us, this way 39 + 28.
+  p.flat = Cin % 64 == 0;
+  int bn = Cin <= 128 ? 128 : 256;
+  if (p.flat) {
+    const int blocks = p.taps * (Cin / 64), fewest = (blocks + 3) / 4;
+    bn = 64;
+    while ((blocks + bn / 64 - 1) / (bn / 64) > fewest) bn += 64;
+  }
+  const int cols = p.flat ? p.taps * Cin : Cin;
+  const long long base_tiles =
+      static_cast<long long>((Cout + kConvBM - 1) / kConvBM) * ((cols + bn - 1) / bn) * (p.flat ? 1 : p.taps);
   const long long pix_tiles = static_cast<long long>(p.tiles_w) * p.tiles_h * p.tiles_n;
   // Split of the pixel loop with the fewest k-blocks on the longest CTA: rounds of one tile per SM, each as long as its
   // k-blocks plus about eight for filling the pipeline and adding the tile into dW.
@@ -633,6 +665,8 @@ MSB_EXPORT int MSB_FN(msb_conv_wgrad)(const void* x, const void* dy, float* dw, 
     MSB_CUDA_CHECK(cudaMemsetAsync(dw, 0, sizeof(float) * static_cast<size_t>(Cout) * R * S * Cin, stream));
   const long long tiles = base_tiles * split;
   if (bn == 256) return launch_conv<256, true>(maps, tmDY, tmY, p, (int)tiles, stream);
+  if (bn == 192) return launch_conv<192, true>(maps, tmDY, tmY, p, (int)tiles, stream);
+  if (bn == 64) return launch_conv<64, true>(maps, tmDY, tmY, p, (int)tiles, stream);
   return launch_conv<128, true>(maps, tmDY, tmY, p, (int)tiles, stream);
 }
 

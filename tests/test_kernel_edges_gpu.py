@@ -261,7 +261,8 @@ def test_gemm_cta_pair_batched(K, a_mn, b_mn, M, N, Kd, dtype):
 
 # ------------------------------------------------------------------------------------------------ convolution
 @pytest.mark.parametrize("N,C,H,W,Cout,k,stride", [(1, 64, 7, 7, 64, 3, 1), (3, 64, 13, 9, 256, 1, 1),
-                                                  (2, 128, 15, 15, 128, 3, 2), (5, 64, 3, 5, 320, 1, 1)])
+                                                  (2, 128, 15, 15, 128, 3, 2), (5, 64, 3, 5, 320, 1, 1),
+                                                  (2, 320, 9, 6, 72, 1, 1), (1, 64, 9, 21, 200, 3, 1)])
 def test_convolution_edges(K, N, C, H, W, Cout, k, stride):
     """Pixel tiles that overhang the image on every side, one and several column blocks: output, the statistics that the
     epilogue gathers, and the weight gradient."""
