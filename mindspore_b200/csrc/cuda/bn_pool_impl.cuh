@@ -186,12 +186,16 @@ bn_apply_kernel(const elem_t* __restrict__ x, const float* __restrict__ scale, c
 }
 
 // dx = gamma * rstd * (dy' - sum(dy')/count - xhat * sum(dy' xhat)/count) = A[c] * dy' + B[c] * x + D[c];
-// dres = dy' (optional).  coef = [A | B | D], each C floats.
+// dres = dy' (optional).  coef = [A | B | D], each C floats.  dgamma and dbeta (optional) are the two sums in the 16-bit type:
+// as casts of their own they were two launches of each layer, which cost the host more than the kernels.
 __global__ void bn_bwd_coeff_kernel(const void* __restrict__ gamma, int affine16, const float* __restrict__ mean,
                                     const float* __restrict__ rstd, const float* __restrict__ sums,
-                                    float* __restrict__ coef, int C, float inv_count) {
+                                    float* __restrict__ coef, elem_t* __restrict__ dgamma, elem_t* __restrict__ dbeta,
+                                    int C, float inv_count) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
+  if (dgamma) dgamma[c] = f_to_e(sums[C + c]);
+  if (dbeta) dbeta[c] = f_to_e(sums[c]);
   const float g = affine(gamma, c, affine16), r = rstd[c], mu = mean[c];
   const float s1 = sums[c] * inv_count, s2 = sums[C + c] * inv_count;
   coef[c] = g * r;
@@ -432,12 +436,12 @@ MSB_EXPORT int MSB_FN(msb_bn_bwd_reduce)(const void* dy, const void* x, const vo
 
 // coef: fp32 [3C] scratch owned by the caller (filled here).
 MSB_EXPORT int MSB_FN(msb_bn_bwd_apply)(const void* dy, const void* x, const void* y, const void* gamma, int affine16, const float* mean,
-                                const float* rstd, const float* sums, float* coef, void* dx, void* dres,
-                                long long rows, int C, int relu, void* stream) {
+                                const float* rstd, const float* sums, float* coef, void* dgamma, void* dbeta,
+                                void* dx, void* dres, long long rows, int C, int relu, void* stream) {
   if (int rc = check_c("bn_bwd_apply", C)) return rc;
   if (rows <= 0) return kOk;
-  bn_bwd_coeff_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(gamma, affine16, mean, rstd, sums, coef, C,
-                                                                         1.f / (float)rows);
+  bn_bwd_coeff_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(gamma, affine16, mean, rstd, sums, coef,
+                                                                         (elem_t*)dgamma, (elem_t*)dbeta, C, 1.f / (float)rows);
   const long long tv = rows * (C / 8);
   bn_bwd_apply_kernel<<<ew_grid((tv + 1) / 2), kEwThreads, 0, (cudaStream_t)stream>>>(
       (const elem_t*)dy, (const elem_t*)x, (const elem_t*)y, coef, (elem_t*)dx,

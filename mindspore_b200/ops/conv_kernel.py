@@ -27,7 +27,7 @@ _native.register_cuda_signature("msb_channel_stats", _I, [_P, _P, _L, _I, _P])
 _native.register_cuda_signature("msb_bn_finalize", _I, [_P] * 3 + [_I] + [_P] * 6 + [_I, _F, _F, _F, _I, _P])
 _native.register_cuda_signature("msb_bn_apply", _I, [_P, _P, _P, _P, _P, _L, _I, _I, _P])
 _native.register_cuda_signature("msb_bn_bwd_reduce", _I, [_P, _P, _P, _P, _P, _P, _L, _I, _I, _P])
-_native.register_cuda_signature("msb_bn_bwd_apply", _I, [_P] * 4 + [_I] + [_P] * 6 + [_L, _I, _I, _P])
+_native.register_cuda_signature("msb_bn_bwd_apply", _I, [_P] * 4 + [_I] + [_P] * 8 + [_L, _I, _I, _P])
 _native.register_cuda_signature("msb_maxpool3x3s2", _I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P])
 _native.register_cuda_signature("msb_global_avgpool", _I, [_P, _P, _I, _I, _I, _I, _P])
 
@@ -263,11 +263,15 @@ class _BnActFn(torch.autograd.Function):
         dx = torch.empty_like(x, memory_format=CL)
         dres = torch.empty_like(x, memory_format=CL) if ctx.has_res else None
         coef = torch.empty(3 * c, dtype=torch.float32, device=x.device)
+        # affine parameters of x's type get their gradients from the kernel, unless they are accumulated elsewhere
+        own = [ctx.affine16 and rows > 0 and getattr(ref, "main_grad", None) is None for ref in (ctx.gamma_ref, ctx.beta_ref)]
+        dgamma, dbeta = (torch.empty(c, dtype=x.dtype, device=x.device) if o else None for o in own)
         _native.check(K._fn("msb_bn_bwd_apply", x)(_p(dy), _p(x), _p(y), _p(g), ctx.affine16, _p(mean), _p(rstd), _p(sums),
-                                                    _p(coef), _p(dx), _p(dres), rows, c, int(ctx.relu), _stream()),
+                                                    _p(coef), _p(dgamma), _p(dbeta), _p(dx), _p(dres), rows, c,
+                                                    int(ctx.relu), _stream()),
                       "bn_bwd_apply")
         _count(3)
-        dgamma, dbeta = sums[c:], sums[:c]
+        dgamma, dbeta = dgamma if own[0] else sums[c:], dbeta if own[1] else sums[:c]
         out_g = out_b = None
         for ref, g, slot in ((ctx.gamma_ref, dgamma, 0), (ctx.beta_ref, dbeta, 1)):
             mg = getattr(ref, "main_grad", None)

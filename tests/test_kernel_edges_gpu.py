@@ -280,3 +280,20 @@ def test_convolution_edges(K, N, C, H, W, Cout, k, stride):
     refw = torch.nn.grad.conv2d_weight(x.double(), w.shape, dy.double(), stride, k // 2)
     _near(dw, refw, 1024, torch.float32)
     _status_ok()
+
+
+def test_batch_norm_affine_gradients(K):
+    """Gradients of 16-bit gamma and beta, which the backward kernel writes itself."""
+    from mindspore_b200.ops import conv_kernel as CK
+    N, C, H, W = 3, 72, 5, 7
+    x = torch.randn(N, C, H, W, device=DEV).bfloat16().to(memory_format=torch.channels_last)
+    xd = x.double()
+    stats = torch.cat([xd.sum((0, 2, 3)), xd.pow(2).sum((0, 2, 3))]).float()
+    gamma, beta = ((torch.randn(C, device=DEV) * 0.1 + o).bfloat16().requires_grad_() for o in (1, 0))
+    y = CK._BnActFn.apply(x, stats, gamma, beta, None, False, 1e-5, (torch.zeros(C, device=DEV), torch.ones(C, device=DEV), 0.9))
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    xhat = (xd - xd.mean((0, 2, 3), keepdim=True)) * torch.rsqrt(xd.var((0, 2, 3), unbiased=False, keepdim=True) + 1e-5)
+    _near(gamma.grad, (dy.double() * xhat).sum((0, 2, 3)), 2, torch.bfloat16)
+    _near(beta.grad, dy.double().sum((0, 2, 3)), 2, torch.bfloat16)
+    _status_ok()
