@@ -86,7 +86,8 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tmap, const
                : "memory");
 }
 
-template <int BN, bool WGRAD>
+// B_MN: B is read MN-major (always in the weight gradient; in the data gradient, whose weights are [k, tap, n]).
+template <int BN, bool WGRAD, bool B_MN>
 __global__ void __launch_bounds__(kConvThreads, 1)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant__ CUtensorMap tmX1,
                   const __grid_constant__ CUtensorMap tmX2, const __grid_constant__ CUtensorMap tmX3,
@@ -198,9 +199,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
         // not loaded (its rows and columns of the product are not stored either)
         const CUtensorMap* bx[BN / 64];
         int bc[BN / 64], bh[BN / 64], bw[BN / 64], a_blocks = 2, b_blocks = BN / 64;
+        if (B_MN) b_blocks = min(BN / 64, (gemm_n - nc0 + 63) / 64);
         if (WGRAD) {
           a_blocks = min(2, (p.Cout - m_blk * kConvBM + 63) / 64);
-          b_blocks = min(BN / 64, (gemm_n - nc0 + 63) / 64);
 #pragma unroll
           for (int j = 0; j < BN / 64; ++j) {
             const int col = min(nc0 + 64 * j, gemm_n - 1);
@@ -211,7 +212,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
             bw[j] = p.tap_dw[tap];
           }
         }
-        const int stage_bytes = WGRAD ? (a_blocks + b_blocks) * 8192 : Cfg::kStageBytes;
+        const int stage_bytes = (a_blocks + b_blocks) * 8192;
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           if (!mbar_wait(&empty_bar[s], ph ^ 1, ab)) { ok = false; break; }
           mbar_expect_tx(&full_bar[s], stage_bytes);
@@ -231,7 +232,14 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
             const int cb = kb - tap * p.cin_blocks;
             tma_load_4d(a_dst, maps[p.tap_map[tap]], &full_bar[s], cb * 64, w0 + p.tap_dw[tap], h0 + p.tap_dh[tap],
                         n0);
-            tma_load_3d(b_dst, &tmO, &full_bar[s], kb * kConvBK, nc0, 0);
+            if (B_MN) {
+#pragma unroll
+              for (int j = 0; j < BN / 64; ++j)
+                if (j < b_blocks)
+                  tma_load_3d(b_dst + j * 8192, &tmO, &full_bar[s], tap * p.Cout + nc0 + 64 * j, cb * 64, 0);
+            } else {
+              tma_load_3d(b_dst, &tmO, &full_bar[s], kb * kConvBK, nc0, 0);
+            }
           }
           ++issued;
           *issued_cnt = issued;
@@ -242,10 +250,10 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer (whole warp, one elected lane)
-    constexpr uint32_t idesc = umma_idesc_elem(kConvBM, BN, WGRAD, WGRAD);
+    constexpr uint32_t idesc = umma_idesc_elem(kConvBM, BN, WGRAD, B_MN);
     const uint32_t lead = elect_one();
     const uint64_t a_desc = umma_smem_desc(smem_u32(smem_a), WGRAD ? 8192 : 16, 1024);
-    const uint64_t b_desc = umma_smem_desc(smem_u32(smem_b), WGRAD ? 8192 : 16, 1024);
+    const uint64_t b_desc = umma_smem_desc(smem_u32(smem_b), B_MN ? 8192 : 16, 1024);
     int s = 0;
     uint32_t ph = 0;
     int it = 0;
@@ -269,7 +277,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constan
           *consumed_cnt = consumed;
 #pragma unroll
           for (int kk = 0; kk < kConvBK / 16; ++kk)
-            umma_bf16(d_tmem, ad + kk * (WGRAD ? 128 : 2), bd + kk * (WGRAD ? 128 : 2), idesc, (kb != kb_lo) || (kk != 0));
+            umma_bf16(d_tmem, ad + kk * (WGRAD ? 128 : 2), bd + kk * (B_MN ? 128 : 2), idesc, (kb != kb_lo) || (kk != 0));
           umma_commit(&empty_bar[s]);
         }
         __syncwarp();
@@ -539,11 +547,11 @@ int setup_input(CUtensorMap maps[4], ConvParams* p, const void* x, int N, int H,
   return kOk;
 }
 
-template <int BN, bool WGRAD>
+template <int BN, bool WGRAD, bool B_MN = WGRAD>
 int launch_conv(const CUtensorMap maps[4], const CUtensorMap& tmO, const CUtensorMap& tmY, const ConvParams& p, int tiles,
                 cudaStream_t stream) {
   using Cfg = ConvCfg<BN>;
-  auto kern = conv_igemm_kernel<BN, WGRAD>;
+  auto kern = conv_igemm_kernel<BN, WGRAD, B_MN>;
   static bool configured = false;
   if (!configured) {
     MSB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes));
@@ -561,6 +569,8 @@ int launch_conv(const CUtensorMap maps[4], const CUtensorMap& tmO, const CUtenso
 // flip = 0: y[ho, wo] += x[ho*stride + r - pad_h, wo*stride + s - pad_w] * w[r, s]      (forward)
 // flip = 1: y[ho, wo] += x[ho + pad_h - r, wo + pad_w - s] * w[r, s]  (stride 1 only)   (data gradient, with
 //           x = dY, w = weights permuted to [Cin, R, S, Cout])
+// flip = 2: as 1 with w as the forward pass holds it, which is [Cin, R, S, Cout] in the terms of this call: no permuted copy
+//           of the weights, one launch less per layer (Cout a multiple of 8)
 // stats (optional): fp32 [2 * Cout], += per-channel sum and sum of squares of y (caller zeroes it).
 // Cin must be a multiple of 64.
 MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float* stats, int N, int H, int W, int Cin,
@@ -572,6 +582,7 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
     return kBadArg;
   }
   if (flip && stride != 1) { set_last_error("conv_fwd: the data-gradient form needs stride 1"); return kBadArg; }
+  if (flip == 2 && (Cout % 8)) { set_last_error("conv_fwd: data gradient of %d channels (multiple of 8)", Cout); return kBadArg; }
   if (stats && (Cout > kMaxStatChannels || out_fp32)) {
     set_last_error("conv_fwd: fused statistics need bf16 output and at most %d channels", kMaxStatChannels);
     return kBadArg;
@@ -590,7 +601,13 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
   // 1x1 256 -> 64 and 3x3 64 -> 64, forward and data gradient: 172 -> 139 us).
   const int bn = Cout <= 64 ? 64 : (Cout <= 128 || pix_tiles * ((Cout + 255) / 256) < sm_count()) ? 128 : 256;
   const long long K = static_cast<long long>(R) * S * Cin;
-  if (int rc = encode_tmap_3d(&tmW, w, 2, K, Cout, 1, K * 2, K * 2 * Cout, 64, bn, 1)) return rc;
+  const bool b_mn = flip == 2;
+  if (b_mn) {
+    const long long row = static_cast<long long>(R) * S * Cout;
+    if (int rc = encode_tmap_3d(&tmW, w, 2, row, Cin, 1, row * 2, row * 2 * Cin, 64, 64, 1)) return rc;
+  } else {
+    if (int rc = encode_tmap_3d(&tmW, w, 2, K, Cout, 1, K * 2, K * 2 * Cout, 64, bn, 1)) return rc;
+  }
   // the output as TMA sees it: a warp's 32 rows are a sub-box of the tile's (all extents are powers of two)
   CUtensorMap tmY = tmW;
   if (!out_fp32 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && ldy % 8 == 0) {
@@ -604,6 +621,11 @@ MSB_EXPORT int MSB_FN(msb_conv_fwd)(const void* x, const void* w, void* y, float
   const long long tiles = pix_tiles * ((Cout + bn - 1) / bn);
   if (tiles > 0x7fffffffLL) { set_last_error("conv_fwd: too many tiles"); return kTooLarge; }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (b_mn) {
+    if (bn == 256) return launch_conv<256, false, true>(maps, tmW, tmY, p, (int)tiles, stream);
+    if (bn == 64) return launch_conv<64, false, true>(maps, tmW, tmY, p, (int)tiles, stream);
+    return launch_conv<128, false, true>(maps, tmW, tmY, p, (int)tiles, stream);
+  }
   if (bn == 256) return launch_conv<256, false>(maps, tmW, tmY, p, (int)tiles, stream);
   if (bn == 64) return launch_conv<64, false>(maps, tmW, tmY, p, (int)tiles, stream);
   return launch_conv<128, false>(maps, tmW, tmY, p, (int)tiles, stream);

@@ -75,9 +75,12 @@ def _w_krsc(w):
 
 # ------------------------------------------------------------------------------------------------ raw launches
 def conv_fwd_raw(x, w_krsc, stride, pad_h, pad_w, ho, wo, stats=None, flip=False):
-    """x NHWC-memory [N, Cin, H, W]; w_krsc [Cout, R, S, Cin] -> y [N, Cout, ho, wo] (channels-last)."""
+    """x NHWC-memory [N, Cin, H, W]; w_krsc [Cout, R, S, Cin] -> y [N, Cout, ho, wo] (channels-last).  ``flip``: 1 for the
+    data gradient, 2 for it with the weights of the forward pass, [Cin, R, S, Cout] here."""
     n, cin, h, w_ = x.shape
-    cout, r, s, _ = w_krsc.shape
+    cout, r, s, last = w_krsc.shape
+    if flip == 2:
+        cout = last
     y = _empty(n, cout, ho, wo, x.device, x.dtype)
     rc = K._fn("msb_conv_fwd", x)(_p(x), _p(w_krsc), _p(y), _p(stats), n, h, w_, cin, cout, r, s, stride, pad_h,
                                      pad_w, int(flip), ho, wo, cin, cout, 0, _stream())
@@ -141,7 +144,7 @@ class _ConvFn(torch.autograd.Function):
                 _count()
         else:
             y = conv_fwd_raw(x, wk, stride, pad_h, pad_w, ho, wo, stats)
-        ctx.save_for_backward(x, w)
+        ctx.save_for_backward(x, w, None if ctx.small else wk)
         ctx.col = (col, kpad) if ctx.small else None      # the patch matrix is kept for the weight gradient
         ctx.geom = (stride, pad_h, pad_w, ho, wo)
         if want_stats:
@@ -152,7 +155,7 @@ class _ConvFn(torch.autograd.Function):
     @staticmethod
     @_quietly
     def backward(ctx, dy, _dstats):
-        x, w = ctx.saved_tensors
+        x, w, wt = ctx.saved_tensors
         stride, pad_h, pad_w, ho, wo = ctx.geom
         n, cin, h, w_ = x.shape
         cout, _, r, s = w.shape
@@ -181,23 +184,24 @@ class _ConvFn(torch.autograd.Function):
                 raise NotImplementedError("data gradient of a convolution with fewer than 64 input channels on the "
                                           "kernel path (only a first layer, whose input needs no gradient, is "
                                           "expected)")
-            wt = w.permute(1, 2, 3, 0).contiguous()                      # [Cin, R, S, Cout]
+            flip = 2
             if cout % 64:                                                # the box loads take 64 channels at a time
+                flip, wt = 1, w.permute(1, 2, 3, 0).contiguous()         # [Cin, R, S, Cout]
                 extra = 64 - cout % 64
                 wt = torch.nn.functional.pad(wt, (0, extra))
                 dy = _nhwc(torch.nn.functional.pad(dy, (0, 0, 0, 0, 0, extra)))
                 cout += extra
             if stride == 1:
-                dx = conv_fwd_raw(dy, wt, 1, pad_h, pad_w, h, w_, None, flip=True)
+                dx = conv_fwd_raw(dy, wt, 1, pad_h, pad_w, h, w_, None, flip=flip)
             elif r == 1 and s == 1:
-                sub = conv_fwd_raw(dy, wt, 1, 0, 0, ho, wo, None, flip=True)
+                sub = conv_fwd_raw(dy, wt, 1, 0, 0, ho, wo, None, flip=flip)
                 dx = _empty(n, cin, h, w_, dy.device, dy.dtype).zero_()
                 dx[:, :, 0:2 * ho:2, 0:2 * wo:2] = sub
             else:
                 hz, wz = max(h, 2 * (ho - 1) + 1), max(w_, 2 * (wo - 1) + 1)
                 dyz = _empty(n, cout, hz, wz, dy.device, dy.dtype).zero_()
                 dyz[:, :, 0:2 * ho:2, 0:2 * wo:2] = dy
-                dx = conv_fwd_raw(dyz, wt, 1, pad_h, pad_w, h, w_, None, flip=True)
+                dx = conv_fwd_raw(dyz, wt, 1, pad_h, pad_w, h, w_, None, flip=flip)
         return dx, dw, None, None, None, None
 
 

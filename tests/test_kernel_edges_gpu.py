@@ -282,6 +282,22 @@ def test_convolution_edges(K, N, C, H, W, Cout, k, stride):
     _status_ok()
 
 
+@pytest.mark.parametrize("N,C,H,W,Cout,k,stride", [(1, 64, 7, 7, 64, 3, 1), (2, 320, 5, 9, 64, 3, 1), (38, 192, 28, 28, 64, 1, 1),
+                                                  (3, 128, 8, 6, 320, 1, 2), (2, 128, 9, 9, 192, 3, 2), (2, 64, 9, 9, 72, 3, 1)])
+def test_convolution_data_gradient(K, N, C, H, W, Cout, k, stride):
+    """The data gradient by the weights of the forward pass in their own order (72 channels: a padded copy), one and several
+    column blocks, strides included."""
+    from mindspore_b200.ops import conv_kernel as CK
+    x = torch.randn(N, C, H, W, device=DEV).bfloat16().to(memory_format=torch.channels_last).requires_grad_()
+    w = (torch.randn(Cout, C, k, k, device=DEV) / math.sqrt(C * k * k)).bfloat16()
+    y, _ = CK._ConvFn.apply(x, w, stride, k // 2, k // 2, False)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    ref = torch.nn.grad.conv2d_input(x.shape, w.double(), dy.double(), stride, k // 2)
+    _near(x.grad, ref, 2, torch.bfloat16)
+    _status_ok()
+
+
 def test_batch_norm_affine_gradients(K):
     """Gradients of 16-bit gamma and beta, which the backward kernel writes itself."""
     from mindspore_b200.ops import conv_kernel as CK
